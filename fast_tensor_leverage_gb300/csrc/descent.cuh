@@ -4,9 +4,9 @@
 // A descent for query x evaluates x^T G x against node Grams.  With the
 // packed upper triangle of G and the packed weighted outer product
 // xx_e = (2 - [a==b]) x_a x_b, the form is a plain dot product over
-// P = R(R+1)/2 values, so a warp holds xx in registers (R <= 32: 17 values
-// per lane) or in its shared-memory slot (R > 32) for the whole descent and
-// every level costs P coalesced loads, P FMAs and one warp reduction.
+// P = R(R+1)/2 values, so a warp keeps xx in its shared-memory slot for the
+// whole descent and every level costs P coalesced loads, P FMAs and one warp
+// reduction.
 //
 // Two arithmetics:
 //   * FP64 (parity mode): exactly the reference's decisions,
@@ -26,9 +26,6 @@
 #ifndef FTL_DESC_PREFETCH
 #define FTL_DESC_PREFETCH 0        // L2 prefetch of next-level candidates (measured slower)
 #endif
-#ifndef FTL_DESC_XX_SMEM32
-#define FTL_DESC_XX_SMEM32 1       // keep the outer product in shared memory also for R <= 32
-#endif
 #ifndef FTL_DESC_EVAL2
 #define FTL_DESC_EVAL2 1           // root and first-level forms in one round trip
 #endif
@@ -44,12 +41,6 @@
 #ifndef FTL_DESC_REDO
 #define FTL_DESC_REDO 1            // FP32: flag samples that met a zero-mass block for the careful redo
 #endif
-#ifndef FTL_DESC_RESIDENT_F32
-#define FTL_DESC_RESIDENT_F32 1536 // threads per SM the FP32 kernels are register-budgeted for
-#endif
-#ifndef FTL_DESC_RESIDENT_F64
-#define FTL_DESC_RESIDENT_F64 512
-#endif
 #ifndef FTL_DESC_WARPS_D32
 #define FTL_DESC_WARPS_D32 4       // FP32 DIAG32 packed (multi-request) draws and tree sampler: warps per block
 #endif
@@ -64,7 +55,6 @@ struct Shape {
     static constexpr int PMAX = RMAX * (RMAX + 1) / 2;
     static constexpr int XPL = (RMAX + 31) / 32;  // vector entries per lane
     static constexpr int FQ = (RMAX + 31) / 32;   // leaf rows per lane (F <= R)
-    static constexpr bool XX_SMEM = RMAX > 32 || FTL_DESC_XX_SMEM32;
     static constexpr int WARPS = RMAX <= 32 ? FTL_DESC_WARPS32 : (RMAX <= 64 ? 4 : 2);
 };
 
@@ -117,127 +107,94 @@ struct NodeShape {
 // plus the packed outer product when it does not fit in registers.
 template <int RMAX, typename T, bool DIAG = false>
 struct WarpSlot {
-    static constexpr size_t xx_elems = (Shape<RMAX>::XX_SMEM && !DIAG) ? NodeShape<RMAX, T>::SMAX : 0;
+    static constexpr size_t xx_elems = DIAG ? 0 : NodeShape<RMAX, T>::SMAX;
     static constexpr size_t bytes =
         ((RMAX * sizeof(double) + RMAX * sizeof(T) + xx_elems * sizeof(T)) + 15) / 16 * 16;
 };
 
 // x^T G x for one query x against any node G (packed, node stride S): the
 // node is read as 16-byte vectors, vector v of lane l is v = l + 32 t, and
-// the matching weighted outer-product values live in registers (R <= 32) or
-// in the warp's shared-memory slot.
+// the matching weighted outer-product values live in the warp's shared-memory
+// slot.
 template <int RMAX, typename T>
 struct QForm {
-    using S_ = Shape<RMAX>;
     using NS = NodeShape<RMAX, T>;
     using V = typename Vec16<T>::type;
     static constexpr int W = NS::W;
-    T r[S_::XX_SMEM ? 1 : NS::NV * W];
     T *s;
     int P, S;
 
     __device__ __forceinline__ void setup(const T *x, const uint16_t *pairs, int lane) {
-        if (S_::XX_SMEM) {
-            for (int e = lane; e < S; e += 32) {
-                T v = T(0);
-                if (e < P) {
-                    unsigned pr = pairs[e];
-                    int a = pr >> 8, b = pr & 0xff;
-                    v = x[a] * x[b];
-                    if (a != b) v += v;
-                }
-                s[e] = v;
+        for (int e = lane; e < S; e += 32) {
+            T v = T(0);
+            if (e < P) {
+                unsigned pr = pairs[e];
+                int a = pr >> 8, b = pr & 0xff;
+                v = x[a] * x[b];
+                if (a != b) v += v;
             }
-            __syncwarp();
-        } else {
+            s[e] = v;
+        }
+        __syncwarp();
+    }
+
+    // Node vectors a lane loads before it uses any of them.  A node of R = 64
+    // is 8.3 KB (FP32): 17 vectors per lane, and with two in flight a level
+    // cost nine dependent L2 round trips.  N = 4, R = 64, J = 32,768 FP32
+    // draw: 7.24 ms with 2, 4.50 ms with 8 (640 threads per SM), 3.83 ms with
+    // all 17 (512 threads).  R <= 32 keeps 2: five or nine vectors, many warps.
+    static constexpr int LB = RMAX <= 32 ? 2 : (sizeof(T) == 8 ? 8 : (RMAX <= 64 ? 17 : 32));
+
+    // acc + this lane's products of its vectors t0 .. t0 + LB - 1, in the
+    // order of the elements; FULL: all of them lie inside the node
+    template <bool FULL>
+    static __device__ __forceinline__ T batch(T acc, const T *__restrict__ node, const T *s, int S, int t0, int lane) {
+        const int e0 = (lane + 32 * t0) * W;
+        V g[LB];
 #pragma unroll
-            for (int t = 0; t < NS::NV; ++t) {
+        for (int u = 0; u < LB; ++u)
+            if (FULL || e0 + 32 * W * u < S) g[u] = __ldg(reinterpret_cast<const V *>(node + e0 + 32 * W * u));
 #pragma unroll
-                for (int w = 0; w < W; ++w) {
-                    int e = (lane + 32 * t) * W + w;
-                    T v = T(0);
-                    if (e < P) {
-                        unsigned pr = pairs[e];
-                        int a = pr >> 8, b = pr & 0xff;
-                        v = x[a] * x[b];
-                        if (a != b) v += v;
-                    }
-                    r[t * W + w] = v;
-                }
+        for (int u = 0; u < LB; ++u) {
+            if (FULL || e0 + 32 * W * u < S) {
+                T gv[W], xv[W];
+                Vec16<T>::get(g[u], gv);
+                Vec16<T>::get(*reinterpret_cast<const V *>(s + e0 + 32 * W * u), xv);
+#pragma unroll
+                for (int w = 0; w < W; ++w) acc = fma(gv[w], xv[w], acc);
             }
         }
+        return acc;
+    }
+
+    // This lane's part of the form.  Large nodes: one copy of the code, called;
+    // inlined at every level and root, the loads of two forms were scheduled
+    // together and spilled (200 registers at R = 64 instead of 96).
+    static constexpr bool CALL = RMAX > 32;
+    __device__ __forceinline__ T partial(const T *__restrict__ node, int lane) const {
+        if constexpr (CALL) return partial_call(node, s, S, lane);
+        else return partial_of(node, s, S, lane);
+    }
+    static __device__ __noinline__ T partial_call(const T *node, const T *s, int S, int lane) {
+        return partial_of(node, s, S, lane);
+    }
+    static __device__ __forceinline__ T partial_of(const T *__restrict__ node, const T *s, int S, int lane) {
+        const int full = S / (32 * W);  // vectors every lane has
+        T acc = T(0);
+        int t = 0;
+#pragma unroll 1
+        for (; t + LB <= full; t += LB) acc = batch<true>(acc, node, s, S, t, lane);
+        return batch<false>(acc, node, s, S, t, lane);
     }
 
     __device__ __forceinline__ T eval(const T *__restrict__ node, int lane) const {
-        T acc = T(0);
-        if (S_::XX_SMEM) {
-#pragma unroll(NS::NV <= 8 ? NS::NV : 2)
-            for (int t = 0; t < NS::NV; ++t) {
-                int e = (lane + 32 * t) * W;
-                if (e < S) {
-                    V g = __ldg(reinterpret_cast<const V *>(node + e));
-                    V x = *reinterpret_cast<const V *>(s + e);
-                    T gv[W], xv[W];
-                    Vec16<T>::get(g, gv);
-                    Vec16<T>::get(x, xv);
-#pragma unroll
-                    for (int w = 0; w < W; ++w) acc = fma(gv[w], xv[w], acc);
-                }
-            }
-        } else {
-#pragma unroll
-            for (int t = 0; t < NS::NV; ++t) {
-                int e = (lane + 32 * t) * W;
-                if (e < S) {
-                    V g = __ldg(reinterpret_cast<const V *>(node + e));
-                    T gv[W];
-                    Vec16<T>::get(g, gv);
-#pragma unroll
-                    for (int w = 0; w < W; ++w) acc = fma(gv[w], r[t * W + w], acc);
-                }
-            }
-        }
-        return warp_sum(acc);
+        return warp_sum(partial(node, lane));
     }
 
     // Two independent forms with interleaved loads (one memory round trip).
     __device__ __forceinline__ void eval2(const T *__restrict__ na, const T *__restrict__ nb,
                                           int lane, T &ra, T &rb) const {
-        T acc_a = T(0), acc_b = T(0);
-        if (S_::XX_SMEM) {
-#pragma unroll 2
-            for (int e = lane * W; e < S; e += 32 * W) {
-                V ga = __ldg(reinterpret_cast<const V *>(na + e));
-                V gb = __ldg(reinterpret_cast<const V *>(nb + e));
-                V x = *reinterpret_cast<const V *>(s + e);
-                T av[W], bv[W], xv[W];
-                Vec16<T>::get(ga, av);
-                Vec16<T>::get(gb, bv);
-                Vec16<T>::get(x, xv);
-#pragma unroll
-                for (int w = 0; w < W; ++w) {
-                    acc_a = fma(av[w], xv[w], acc_a);
-                    acc_b = fma(bv[w], xv[w], acc_b);
-                }
-            }
-        } else {
-#pragma unroll
-            for (int t = 0; t < NS::NV; ++t) {
-                int e = (lane + 32 * t) * W;
-                if (e < S) {
-                    V ga = __ldg(reinterpret_cast<const V *>(na + e));
-                    V gb = __ldg(reinterpret_cast<const V *>(nb + e));
-                    T av[W], bv[W];
-                    Vec16<T>::get(ga, av);
-                    Vec16<T>::get(gb, bv);
-#pragma unroll
-                    for (int w = 0; w < W; ++w) {
-                        acc_a = fma(av[w], r[t * W + w], acc_a);
-                        acc_b = fma(bv[w], r[t * W + w], acc_b);
-                    }
-                }
-            }
-        }
+        T acc_a = partial(na, lane), acc_b = partial(nb, lane);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             acc_a += __shfl_xor_sync(0xffffffffu, acc_a, o);

@@ -179,11 +179,15 @@ __device__ __forceinline__ void draw_sample(const DrawParams &p, int64_t i, Draw
     __syncwarp();
 }
 
-// Threads per SM the register budget of a draw kernel is set for.
-template <typename T, bool DIAG>
+// Threads per SM the register budget of a draw kernel is set for: what the
+// warps' outer products leave room for in shared memory (R > 64: one block;
+// 32 < R <= 64: 16 warps in FP32, 12 in FP64), so that the node vectors a
+// warp has in flight get the registers.
+template <int RMAX, typename T, bool DIAG>
 struct Resident {
-    static constexpr int value =
-        sizeof(T) == 8 ? FTL_DESC_RESIDENT_F64 : (DIAG ? FTL_DESC_RESIDENT_D32 : FTL_DESC_RESIDENT_F32);
+    static constexpr int F32 = RMAX <= 32 ? 1536 : (RMAX <= 64 ? 512 : 192);
+    static constexpr int F64 = RMAX <= 32 ? 512 : (RMAX <= 64 ? 384 : 64);
+    static constexpr int value = sizeof(T) == 8 ? F64 : (DIAG ? FTL_DESC_RESIDENT_D32 : F32);
 };
 
 // Samples i0 + c (c < NC, those below J) of one draw for FP32 trees in the
@@ -289,7 +293,7 @@ __device__ __forceinline__ void draw_samples_d32(const DrawParams &p, int64_t i0
 }
 
 template <int RMAX, typename T, bool S32, bool DIAG>
-__global__ void __launch_bounds__(Blk<RMAX, T>::WARPS * 32, Resident<T, DIAG>::value / (Blk<RMAX, T>::WARPS * 32)) krp_draw_kernel(DrawParams p) {
+__global__ void __launch_bounds__(Blk<RMAX, T>::WARPS * 32, Resident<RMAX, T, DIAG>::value / (Blk<RMAX, T>::WARPS * 32)) krp_draw_kernel(DrawParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     DrawWarp<RMAX, T, DIAG> dw;
     setup_draw_warp<RMAX, T, DIAG>(dw, smem_raw, p.R, p.P, p.S);
@@ -381,7 +385,7 @@ __device__ __forceinline__ bool pack_stop(const MultiDrawParams &mp, int r, int 
 }
 
 template <int RMAX, typename T, bool S32, bool DIAG>
-__global__ void __launch_bounds__(Blk<RMAX, T, DIAG>::WARPS * 32, Resident<T, DIAG>::value / (Blk<RMAX, T, DIAG>::WARPS * 32)) krp_draw_multi_kernel(MultiDrawParams mp) {
+__global__ void __launch_bounds__(Blk<RMAX, T, DIAG>::WARPS * 32, Resident<RMAX, T, DIAG>::value / (Blk<RMAX, T, DIAG>::WARPS * 32)) krp_draw_multi_kernel(MultiDrawParams mp) {
     constexpr int WARPS = Blk<RMAX, T, DIAG>::WARPS;
     const int warp = threadIdx.x >> 5;
     const int64_t total = mp.cum[mp.n];
@@ -483,7 +487,7 @@ struct TreeSampleParams {
 // PartitionTree::PTSample_internal (cpp_ext/partition_tree.hpp:232-405):
 // x = scaled_h[i]; samples[i] = selected row; h[i] o= U[row].
 template <int RMAX, typename T, bool DIAG>
-__global__ void __launch_bounds__(Blk<RMAX, T>::WARPS * 32, Resident<T, DIAG>::value / (Blk<RMAX, T>::WARPS * 32)) tree_sample_kernel(TreeSampleParams p) {
+__global__ void __launch_bounds__(Blk<RMAX, T>::WARPS * 32, Resident<RMAX, T, DIAG>::value / (Blk<RMAX, T>::WARPS * 32)) tree_sample_kernel(TreeSampleParams p) {
     using S = Shape<RMAX>;
     constexpr int XPL = S::XPL;
     extern __shared__ __align__(16) unsigned char smem_raw[];
