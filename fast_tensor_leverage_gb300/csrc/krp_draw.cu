@@ -1,7 +1,7 @@
 // Fused KRP leverage-score draw and the standalone tree sampler.
 //
-// krp_draw_kernel: one warp per sample runs, for every included mode k in
-// increasing order, the eigen-component descent (query h) and the Gram-tree
+// krp_draw_kernel (FP32 trees; FP64 trees: krp_draw_fx.cu): one warp per sample
+// runs, for every included mode k in increasing order, the eigen-component descent (query h) and the Gram-tree
 // descent (query h o W[u]) of EfficientKRPSampler::KRPDrawSamples
 // (cpp_ext/efficient_krp_sampler.hpp:209-254), keeping the running KRP row h
 // in registers across modes, then the weight epilogue w = R / (J h^T pinv h)
@@ -14,35 +14,13 @@
 #include <type_traits>
 
 #include "descent.cuh"
+#include "draw_params.cuh"
 
 namespace ftl {
 
 int computem_launch(const ftl_krp_plan *plan, uint32_t j_norm, cudaStream_t st);
 int tuned_variant(int family, int R, int prec);
-
-struct DrawParams {
-    int N, R, P, S;
-    uint32_t j;
-    int64_t J;
-    DGeom gram[FTL_MAX_MODES];
-    DGeom eig;
-    const double *U[FTL_MAX_MODES];
-    const float *U32[FTL_MAX_MODES];  // FP32 copies of U for the leaf scans (S32 kernels)
-    const void *gram_G[FTL_MAX_MODES];
-    const void *eig_G;
-    const double *M;
-    const float *pinv32;
-    int offset[FTL_MAX_MODES];
-    uint64_t *samples;
-    double *h;
-    double *weights;
-    const double *draws;
-    uint64_t seed, ctr;
-};
-
-__device__ __forceinline__ double get_draw(const DrawParams &p, int64_t idx) {
-    return p.draws ? p.draws[idx] : philox_uniform(p.seed, p.ctr + (uint64_t)idx);
-}
+int launch_draw_fx(const DrawParams &p, cudaStream_t st);
 
 // Per-warp state of the draw kernels: the block's pair table and the warp's
 // shared-memory slot.
@@ -292,15 +270,15 @@ __device__ __forceinline__ void draw_samples_d32(const DrawParams &p, int64_t i0
     }
 }
 
-template <int RMAX, typename T, bool S32, bool DIAG>
-__global__ void __launch_bounds__(Blk<RMAX, T>::WARPS * 32, Resident<RMAX, T, DIAG>::value / (Blk<RMAX, T>::WARPS * 32)) krp_draw_kernel(DrawParams p) {
+template <int RMAX, typename T, bool S32>
+__global__ void __launch_bounds__(Blk<RMAX, T>::WARPS * 32, Resident<RMAX, T, false>::value / (Blk<RMAX, T>::WARPS * 32)) krp_draw_kernel(DrawParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    DrawWarp<RMAX, T, DIAG> dw;
-    setup_draw_warp<RMAX, T, DIAG>(dw, smem_raw, p.R, p.P, p.S);
+    DrawWarp<RMAX, T, false> dw;
+    setup_draw_warp<RMAX, T, false>(dw, smem_raw, p.R, p.P, p.S);
     const int warp = threadIdx.x >> 5;
     for (int64_t i = (int64_t)blockIdx.x * Blk<RMAX, T>::WARPS + warp; i < p.J;
          i += (int64_t)gridDim.x * Blk<RMAX, T>::WARPS)
-        draw_sample<RMAX, T, false, S32, DIAG>(p, i, dw);
+        draw_sample<RMAX, T, false, S32, false>(p, i, dw);
 }
 
 // Block shape of the FP32 DIAG32 draw kernel per variant NC (samples a warp
@@ -578,11 +556,12 @@ static int launch_d32(const DrawParams &p, cudaStream_t st) {
     return FTL_OK;
 }
 
-template <int RMAX, typename T, bool S32, bool DIAG>
+template <int RMAX, bool S32, bool DIAG>
 static int launch_draw(const DrawParams &p, cudaStream_t st) {
+    using T = float;
     const int warps = Blk<RMAX, T>::WARPS;
     size_t smem = desc_smem<RMAX, T, DIAG>();
-    if constexpr (FastD32<RMAX, T, DIAG>::value) {
+    if constexpr (DIAG) {
         int lrc;
         switch (tuned_variant(FTL_TUNE_DRAW, p.R, FTL_PREC_FP32)) {
             case 0: lrc = launch_d32<S32, 1, false>(p, st); break;
@@ -594,14 +573,14 @@ static int launch_draw(const DrawParams &p, cudaStream_t st) {
         }
         if (lrc) return lrc;
     } else {
-        const int arc = ensure_smem((const void *)krp_draw_kernel<RMAX, T, S32, DIAG>, smem, "krp_draw_kernel");
+        const int arc = ensure_smem((const void *)krp_draw_kernel<RMAX, T, S32>, smem, "krp_draw_kernel");
         if (arc) return arc;
         int64_t blocks = (p.J + warps - 1) / warps;
         blocks = std::max<int64_t>(1, std::min<int64_t>(blocks, (int64_t)num_sms() * 64));
-        krp_draw_kernel<RMAX, T, S32, DIAG><<<(unsigned)blocks, warps * 32, smem, st>>>(p);
+        krp_draw_kernel<RMAX, T, S32><<<(unsigned)blocks, warps * 32, smem, st>>>(p);
     }
     int rc = check_launch("krp_draw_kernel");
-    if (rc || sizeof(T) == 8) return rc;
+    if (rc) return rc;
     {
         const int arc = ensure_smem((const void *)krp_fixup_kernel<RMAX, S32, DIAG>, smem, "krp_fixup_kernel");
         if (arc) return arc;
@@ -663,21 +642,19 @@ static bool shadows_ready(const DrawParams &p) {
     return true;
 }
 
-template <typename T>
-static int dispatch_draw(const DrawParams &p, cudaStream_t st) {
-    if constexpr (sizeof(T) == 4) {
-        const bool diag = node_layout(p.R, sizeof(T)) == FTL_LAYOUT_DIAG32;
-        if (shadows_ready(p)) {
-            if (diag) return launch_draw<32, T, true, true>(p, st);
-            if (p.R <= 32) return launch_draw<32, T, true, false>(p, st);
-            if (p.R <= 64) return launch_draw<64, T, true, false>(p, st);
-            return launch_draw<128, T, true, false>(p, st);
-        }
-        if (diag) return launch_draw<32, T, false, true>(p, st);
+// FP32 trees.  FP64 trees take launch_draw_fx (krp_draw_fx.cu).
+static int dispatch_draw_f32(const DrawParams &p, cudaStream_t st) {
+    const bool diag = node_layout(p.R, 4) == FTL_LAYOUT_DIAG32;
+    if (shadows_ready(p)) {
+        if (diag) return launch_draw<32, true, true>(p, st);
+        if (p.R <= 32) return launch_draw<32, true, false>(p, st);
+        if (p.R <= 64) return launch_draw<64, true, false>(p, st);
+        return launch_draw<128, true, false>(p, st);
     }
-    if (p.R <= 32) return launch_draw<32, T, false, false>(p, st);
-    if (p.R <= 64) return launch_draw<64, T, false, false>(p, st);
-    return launch_draw<128, T, false, false>(p, st);
+    if (diag) return launch_draw<32, false, true>(p, st);
+    if (p.R <= 32) return launch_draw<32, false, false>(p, st);
+    if (p.R <= 64) return launch_draw<64, false, false>(p, st);
+    return launch_draw<128, false, false>(p, st);
 }
 
 // The register/shared-memory shapes are chosen by max(R, F): a lane handles
@@ -755,8 +732,8 @@ extern "C" int ftl_krp_sample(const ftl_krp_plan *plan, uint32_t j, uint64_t *sa
     DrawParams p;
     fill_draw_params(p, plan, j, samples, h, weights, draws, seed, ctr);
     cudaStream_t st = (cudaStream_t)stream;
-    if (plan->prec == FTL_PREC_FP64) return dispatch_draw<double>(p, st);
-    return dispatch_draw<float>(p, st);
+    if (plan->prec == FTL_PREC_FP64) return launch_draw_fx(p, st);
+    return dispatch_draw_f32(p, st);
 }
 
 static void fill_draw_params(DrawParams &p, const ftl_krp_plan *plan, uint32_t j, uint64_t *samples, double *h,

@@ -1,0 +1,247 @@
+// FP64 KRP draw with certified fixed-point descents (descent_fx.cuh): per
+// sample the steps of krp_draw_kernel<., double> (krp_draw.cu), the decisions
+// of both descents and of the leaf scan from fixed-point and FP32 forms where
+// those are certain, from the FP64 code of descent.cuh where they are not.
+// The FP64 work left per sample is h o W[u], the update of h and the weight.
+//
+// One warp per sample up to R = 64 (at R = 32 a query's outer product takes
+// 4.2 KB of shared memory and 24 warps run per SM); above, a team of four
+// warps shares one sample, since a query of R = 100 takes 40 KB and one warp
+// per sample would leave five warps on an SM.
+#include <algorithm>
+
+#include "descent_fx.cuh"
+
+namespace ftl {
+
+template <int RMAX>
+struct FxShape {
+    static constexpr int TW = RMAX <= 64 ? 1 : 4;          // warps per sample
+    static constexpr int TEAMS = RMAX <= 64 ? 4 : 1;       // samples per block
+    static constexpr int THREADS = 32 * TW * TEAMS;
+    static constexpr int MINB = RMAX <= 32 ? 6 : (RMAX <= 64 ? 3 : 4);  // blocks per SM
+};
+
+// Shared memory of one team, and where its parts lie.
+template <int RMAX>
+struct FxSmem {
+    size_t slot, xd, xs, qrow, red, team;
+    __host__ __device__ explicit FxSmem(int R) {
+        constexpr int ROW = 32 * FxShape<RMAX>::TW;
+        const int nvec = node_stride(R, 8) / 2;
+        size_t o = 0;
+        slot = o;
+        o += (size_t)((nvec + ROW - 1) / ROW * ROW) * sizeof(float4);
+        xd = o;
+        o += RMAX * sizeof(double);
+        xs = o;
+        o += RMAX * sizeof(float2);
+        qrow = o;
+        o += RMAX * sizeof(float);
+        red = o;
+        o += 2 * FxShape<RMAX>::TW * sizeof(int2);
+        team = (o + 15) / 16 * 16;
+    }
+};
+
+// xx of the FP64 form into the team's slot (QForm<., double>::setup's values).
+__device__ __forceinline__ void fx_fill64(double *s, const double *x, int R, int P, int S, int lane) {
+    for (int e = lane; e < S; e += 32) {
+        double v = 0.0;
+        if (e < P) {
+            int a, b;
+            pair_of(e, R, a, b);
+            v = x[a] * x[b];
+            if (a != b) v += v;
+        }
+        s[e] = v;
+    }
+    __syncwarp();
+}
+
+// The FP64 descent (and leaf scan, with_rows) of one sample by one warp; the
+// staged query is in xd, the slot is overwritten.  Returns the row with_rows,
+// else the leaf index.
+template <int RMAX>
+__device__ __noinline__ int64_t fx_redo(const DrawParams &p, const double *G, const DGeom &g, const double *U,
+                                        double *slot, const double *xd, double u, bool with_rows, int lane) {
+    QForm<RMAX, double> qf;
+    qf.P = p.P;
+    qf.S = p.S;
+    qf.s = slot;
+    fx_fill64(slot, xd, p.R, p.P, p.S, lane);
+    double frac;
+    const int64_t c = descend<RMAX>(G, p.S, g, u, qf, lane, frac);
+    if (!with_rows || g.F <= 1) return leaf_index(g, c);
+    bool empty;
+    return leaf_scan<RMAX, double, double>(U, p.R, g, c, frac, lane_query<RMAX, double>(xd, p.R, lane), lane, empty);
+}
+
+template <int RMAX>
+__global__ void __launch_bounds__(FxShape<RMAX>::THREADS, FxShape<RMAX>::MINB) krp_draw_fx_kernel(DrawParams p) {
+    using Sh = FxShape<RMAX>;
+    constexpr int TW = Sh::TW, TEAMS = Sh::TEAMS;
+    constexpr int XPL = Shape<RMAX>::XPL;
+    using Team = FxTeam<RMAX, TW>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int R = p.R, N = p.N, lane = threadIdx.x & 31;
+    const size_t RR = (size_t)R * R;
+    const size_t eig_stride = (size_t)(2 * R - 1) * p.S;
+    int *eg = (int *)smem_raw;  // largest diagonal exponent of the roots: [eigen trees, Gram trees][N]
+    int64_t *answer = (int64_t *)(smem_raw + 2 * FTL_MAX_MODES * sizeof(int));  // TW > 1: a redo's result
+    const FxSmem<RMAX> lay(R);
+    unsigned char *base = smem_raw + 2 * FTL_MAX_MODES * sizeof(int) + 16 + (threadIdx.x / (32 * TW)) * lay.team;
+    Team tm;
+    tm.slot = (float4 *)(base + lay.slot);
+    tm.xd = (double *)(base + lay.xd);
+    tm.xs = (float2 *)(base + lay.xs);
+    tm.qrow = (float *)(base + lay.qrow);
+    tm.red = (int2 *)(base + lay.red);
+    tm.tid = threadIdx.x % (32 * TW);
+    tm.nvec = p.S / 2;
+    tm.fr = tm.nvec / (32 * TW);
+    tm.flip = 0;
+    for (int k = threadIdx.x >> 5; k < 2 * N; k += TW * TEAMS) {
+        const int mode = k % N;
+        unsigned e = 0;
+        if ((uint32_t)mode != p.j) {
+            const double *G = k < N ? (const double *)p.eig_G + mode * eig_stride : (const double *)p.gram_G[mode];
+            for (int a = lane; a < R; a += 32)
+                e = max(e, ((unsigned)__double2hiint(G[packed_row_offset(a, R)]) >> 20) & 0x7ffu);
+        }
+        e = __reduce_max_sync(0xffffffffu, e);
+        if (lane == 0) eg[k] = (int)e;
+    }
+    __syncthreads();
+
+    const int64_t teams = (int64_t)gridDim.x * TEAMS;
+#pragma unroll 1
+    for (int64_t i = (int64_t)blockIdx.x * TEAMS + threadIdx.x / (32 * TW); i < p.J; i += teams) {
+        // lane l < 2N holds uniform l (phase l / N, mode l % N) as 53 bits
+        uint64_t D = 0;
+        bool dok = true;
+        if (lane < 2 * N) {
+            const int64_t idx = (int64_t)lane * p.J + i;
+            if (p.draws) {
+                const double u = p.draws[idx];
+                dok = u >= 0.0 && u < 1.0;
+                if (dok) D = (uint64_t)(u * 9007199254740992.0);
+            } else {
+                D = philox_bits53(p.seed, p.ctr + (uint64_t)idx);
+            }
+        }
+        const unsigned dmask = __ballot_sync(0xffffffffu, dok);
+        double h[XPL];
+#pragma unroll
+        for (int q = 0; q < XPL; ++q) h[q] = 1.0;
+#pragma unroll 1
+        for (int k = 0; k < N; ++k) {
+            if ((uint32_t)k == p.j) continue;
+            double x[XPL];
+#pragma unroll
+            for (int q = 0; q < XPL; ++q) x[q] = lane + 32 * q < R ? h[q] : 0.0;
+#pragma unroll 1
+            for (int phase = 0; phase < 2; ++phase) {
+                const double *G = phase == 0 ? (const double *)p.eig_G + k * eig_stride : (const double *)p.gram_G[k];
+                const DGeom &g = phase == 0 ? p.eig : p.gram[k];
+                const int l = phase * N + k;
+                const uint64_t Dk = __shfl_sync(0xffffffffu, D, l);
+                FxScale sc;
+                FxLeaf lf;
+                bool ok = fx_stage(tm, x, R, eg[l], sc) && ((dmask >> l) & 1u);
+                int64_t t = 0;
+                if (ok) {
+                    if (is_leaf(g, 0)) {  // the leaf fraction is the draw
+                        lf.c = 0;
+                        lf.t = (int64_t)Dk;
+                        lf.m = (int64_t)1 << 53;
+                        lf.tol = lf.mtol = 1;
+                    } else {
+                        ok = fx_descend(tm, G, p.S, g, Dk, sc, lf);
+                    }
+                }
+                if (ok) {
+                    if (phase == 1 && g.F > 1)
+                        ok = fx_leaf_scan(tm, p.U[k], R, g, lf, t);
+                    else
+                        t = leaf_index(g, (int64_t)lf.c);
+                }
+                if (!ok) {
+                    const double u = get_draw(p, (int64_t)l * p.J + i);
+                    Team::sync();
+                    if (TW == 1 || tm.tid < 32) {
+                        t = fx_redo<RMAX>(p, G, g, p.U[k], (double *)tm.slot, tm.xd, u, phase == 1, lane);
+                        if (TW > 1 && lane == 0) *answer = t;
+                    }
+                    Team::sync();
+                    if (TW > 1) t = *answer;
+                    Team::sync();
+                }
+                if (phase == 0) {
+                    const double *Wr = p.M + (size_t)p.offset[k] * RR + (size_t)t * R;
+#pragma unroll
+                    for (int q = 0; q < XPL; ++q) {
+                        const int col = lane + 32 * q;
+                        x[q] = col < R ? h[q] * Wr[col] : 0.0;
+                    }
+                } else {
+                    const double *Ur = p.U[k] + t * R;
+#pragma unroll
+                    for (int q = 0; q < XPL; ++q) {
+                        const int col = lane + 32 * q;
+                        if (col < R) h[q] *= Ur[col];
+                    }
+                    if (tm.tid == 0) p.samples[(int64_t)k * p.J + i] = (uint64_t)t;
+                }
+            }
+        }
+        if (TW == 1 || tm.tid < 32) {
+            if (p.weights) {
+                __syncwarp();
+#pragma unroll
+                for (int q = 0; q < XPL; ++q)
+                    if (lane + 32 * q < R) tm.xd[lane + 32 * q] = h[q];
+                __syncwarp();
+                QForm<RMAX, double> qf;
+                qf.P = p.P;
+                qf.S = p.S;
+                qf.s = (double *)tm.slot;
+                fx_fill64(qf.s, tm.xd, R, p.P, p.S, lane);
+                const double lev = qf.eval(p.M + cm_pinv64_offset(N, R), lane);
+                if (lane == 0) p.weights[i] = (double)R / (lev * (double)p.J);
+            }
+            if (p.h) {
+#pragma unroll
+                for (int q = 0; q < XPL; ++q)
+                    if (lane + 32 * q < R) p.h[i * R + lane + 32 * q] = h[q];
+            }
+        }
+        Team::sync();
+    }
+}
+
+template <int RMAX>
+static int launch_fx(const DrawParams &p, cudaStream_t st) {
+    using Sh = FxShape<RMAX>;
+    const size_t smem = 2 * FTL_MAX_MODES * sizeof(int) + 16 + Sh::TEAMS * FxSmem<RMAX>(p.R).team;
+    int rc = ensure_smem((const void *)krp_draw_fx_kernel<RMAX>, smem, "krp_draw_fx_kernel");
+    if (rc) return rc;
+    // one wave of resident blocks, each looping over samples
+    int occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, krp_draw_fx_kernel<RMAX>, Sh::THREADS, smem) !=
+            cudaSuccess ||
+        occ < 1)
+        occ = 1;
+    const int64_t need = (p.J + Sh::TEAMS - 1) / Sh::TEAMS;
+    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)num_sms() * occ));
+    krp_draw_fx_kernel<RMAX><<<blocks, Sh::THREADS, smem, st>>>(p);
+    return check_launch("krp_draw_fx_kernel");
+}
+
+int launch_draw_fx(const DrawParams &p, cudaStream_t st) {
+    if (p.R <= 32) return launch_fx<32>(p, st);
+    if (p.R <= 64) return launch_fx<64>(p, st);
+    return launch_fx<128>(p, st);
+}
+
+}  // namespace ftl
