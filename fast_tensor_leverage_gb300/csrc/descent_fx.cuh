@@ -56,9 +56,15 @@ __device__ __forceinline__ void fx_split(uint32_t hi, uint32_t lo, int kadj, flo
     const uint32_t sg = hi & 0x80000000u;
     const int a = __viaddmax_s32((int)(hi & 0x7fffffffu), kadj, 0x00100000);
     const uint32_t r = __funnelshift_l(lo, (uint32_t)a, 3);
-    h = __uint_as_float(r | sg);
-    const uint32_t e = (r & 0x7f800000u) | sg;
-    l = __uint_as_float(((lo >> 6) & 0x7fffffu) | e) - __uint_as_float(e);
+    const uint32_t hs = r | sg;
+    h = __uint_as_float(hs);
+    l = __uint_as_float(((lo >> 6) & 0x7fffffu) | (hs & 0xff800000u)) - __uint_as_float(hs & 0xff800000u);
+}
+
+// The upper part alone.
+__device__ __forceinline__ float fx_upper(uint32_t hi, uint32_t lo, int kadj) {
+    const int a = __viaddmax_s32((int)(hi & 0x7fffffffu), kadj, 0x00100000);
+    return __uint_as_float(__funnelshift_l(lo, (uint32_t)a, 3) | (hi & 0x80000000u));
 }
 
 // Scale of one descent: the root's exponent, the accumulators' start and the
@@ -77,6 +83,7 @@ struct FxTeam {
     float2 *xs;    // the scaled query as (upper, lower) FP32 parts
     float *qrow;   // leaf scan: squared forms by row
     int2 *red;     // TW > 1: two sets of per-warp partial sums
+    const uint16_t *pairs;  // per vector: row and column (a << 8 | b) of its first entry
     int tid;       // thread of the team
     int nvec, fr;  // vectors per node; rows of 32 TW vectors that are full
     int flip;
@@ -99,40 +106,48 @@ __device__ __forceinline__ void fx_term(uint32_t hi, uint32_t lo, float xh, floa
     d = fmaf(gl, xh, d);
 }
 
-// The form of the staged query against a node, in units of 2^(k-42).
-template <int RMAX, int TW>
+// The form of the staged query against a node, in units of 2^(k-42).  FR >= 0:
+// the number of full rows, known at compile time (R <= 32; branch-free).
+template <int RMAX, int TW, int FR>
 __device__ __forceinline__ int64_t fx_eval(FxTeam<RMAX, TW> &tm, const double *__restrict__ node, const FxScale &sc) {
     constexpr int ROW = 32 * TW;
     const uint4 *nv = reinterpret_cast<const uint4 *>(node) + tm.tid;
     const float4 *xv = tm.slot + tm.tid;
+    const int fr = FR >= 0 ? FR : tm.fr;
     int hi = 0, lo = 0;
     int u0 = 0;
 #pragma unroll 1
     do {
         uint4 g[kFxCh], gt = make_uint4(0, 0, 0, 0);
-        const bool last = u0 + kFxCh >= tm.fr;
+        const bool last = u0 + kFxCh >= fr, whole = u0 + kFxCh <= fr;
+        if (FR < 0 && whole) {
 #pragma unroll
-        for (int u = 0; u < kFxCh; ++u)
-            if (u0 + u < tm.fr) g[u] = __ldg(nv + (u0 + u) * ROW);
-        if (last && tm.tid + tm.fr * ROW < tm.nvec) gt = __ldg(nv + tm.fr * ROW);
+            for (int u = 0; u < kFxCh; ++u) g[u] = __ldg(nv + (u0 + u) * ROW);
+        } else {
+#pragma unroll
+            for (int u = 0; u < kFxCh; ++u)
+                if (u0 + u < fr) g[u] = __ldg(nv + (u0 + u) * ROW);
+        }
+        if (last && tm.tid + fr * ROW < tm.nvec) gt = __ldg(nv + fr * ROW);
         float s0 = __uint_as_float(sc.cb), s1 = s0, c0 = 0.0f, c1 = 0.0f, d0 = 0.0f, d1 = 0.0f;
+        auto term = [&](const uint4 &v, int u) {
+            const float4 x = xv[u * ROW];
+            fx_term(v.y, v.x, x.x, x.y, sc.kadj, s0, c0, d0);
+            fx_term(v.w, v.z, x.z, x.w, sc.kadj, s1, c1, d1);
+        };
+        if (FR < 0 && whole) {
 #pragma unroll
-        for (int u = 0; u < kFxCh; ++u) {
-            if (u0 + u < tm.fr) {
-                const float4 x = xv[(u0 + u) * ROW];
-                fx_term(g[u].y, g[u].x, x.x, x.y, sc.kadj, s0, c0, d0);
-                fx_term(g[u].w, g[u].z, x.z, x.w, sc.kadj, s1, c1, d1);
-            }
+            for (int u = 0; u < kFxCh; ++u) term(g[u], u0 + u);
+        } else {
+#pragma unroll
+            for (int u = 0; u < kFxCh; ++u)
+                if (u0 + u < fr) term(g[u], u0 + u);
         }
-        if (last && tm.fr * ROW < tm.nvec) {
-            const float4 x = xv[tm.fr * ROW];  // zero past the node
-            fx_term(gt.y, gt.x, x.x, x.y, sc.kadj, s0, c0, d0);
-            fx_term(gt.w, gt.z, x.z, x.w, sc.kadj, s1, c1, d1);
-        }
+        if (last && fr * ROW < tm.nvec) term(gt, fr);  // xx is zero past the node
         hi += (int)(__float_as_uint(s0) - sc.cb) + (int)(__float_as_uint(s1) - sc.cb);
         lo += __float2int_rn(fmaf(d0 + d1, 1.1920928955078125e-07f, c0 + c1) * sc.lscale);
         u0 += kFxCh;
-    } while (u0 < tm.fr);
+    } while (FR < 0 && u0 < fr);
     hi = __reduce_add_sync(0xffffffffu, hi);
     lo = __reduce_add_sync(0xffffffffu, lo);
     if constexpr (TW == 1) {
@@ -153,6 +168,17 @@ __device__ __forceinline__ int64_t fx_eval(FxTeam<RMAX, TW> &tm, const double *_
 template <int RMAX, int TW>
 __device__ __forceinline__ int fx_flushes(const FxTeam<RMAX, TW> &tm) {
     return max(1, (tm.fr + kFxCh - 1) / kFxCh);
+}
+
+// (2 - [a == b]) x_a x_b as an upper and a lower FP32 part.
+__device__ __forceinline__ void fx_product(const float2 *xs, int a, int b, float &ph, float &pl) {
+    const float2 xa = xs[a], xb = xs[b];
+    const float f = a == b ? 1.0f : 2.0f;
+    const float ah = f * xa.x, al = f * xa.y;
+    const float p = ah * xb.x;
+    const float q = fmaf(al, xb.x, fmaf(ah, xb.y, fmaf(ah, xb.x, -p)));
+    ph = p + q;
+    pl = q - (ph - p);
 }
 
 // Stage query x (FP64, XPL entries per lane, every warp of the team holds it)
@@ -190,29 +216,11 @@ __device__ __forceinline__ bool fx_stage(FxTeam<RMAX, TW> &tm, const double (&x)
         const int v = u * ROW + tm.tid;
         float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (2 * v < P) {
-            int a, b;
-            pair_of(2 * v, R, a, b);
-#pragma unroll
-            for (int w = 0; w < 2; ++w) {
-                float ph = 0.0f, pl = 0.0f;
-                if (2 * v + w < P) {
-                    const float2 xa = tm.xs[a], xb = tm.xs[b];
-                    const float f = a == b ? 1.0f : 2.0f;
-                    const float ah = f * xa.x, al = f * xa.y;
-                    const float p = ah * xb.x;
-                    const float q = fmaf(al, xb.x, fmaf(ah, xb.y, fmaf(ah, xb.x, -p)));
-                    ph = p + q;
-                    pl = q - (ph - p);
-                }
-                if (w == 0) {
-                    o.x = ph;
-                    o.y = pl;
-                } else {
-                    o.z = ph;
-                    o.w = pl;
-                }
-                if (++b == R) b = ++a;
-            }
+            const unsigned pr = tm.pairs[v];
+            int a = (int)(pr >> 8), b = (int)(pr & 0xffu);
+            fx_product(tm.xs, a, b, o.x, o.y);
+            if (++b == R) b = ++a;
+            if (2 * v + 1 < P) fx_product(tm.xs, a, b, o.z, o.w);
         }
         tm.slot[v] = o;
         // sums of |xx| per accumulator and flush (the ragged row joins the last)
@@ -248,7 +256,7 @@ struct FxLeaf {
 
 // The descent of descent.cuh's FP64 `descend` for uniform D 2^-53; false when
 // a decision is closer than the error bound.
-template <int RMAX, int TW>
+template <int RMAX, int TW, int FR>
 __device__ __forceinline__ bool fx_descend(FxTeam<RMAX, TW> &tm, const double *__restrict__ G, int S, const DGeom &g,
                                            uint64_t D, const FxScale &sc, FxLeaf &out) {
     const int64_t E = (int64_t)kFxErr * TW * fx_flushes(tm);
@@ -259,7 +267,7 @@ __device__ __forceinline__ bool fx_descend(FxTeam<RMAX, TW> &tm, const double *_
     const double *node = G;
 #pragma unroll 1
     for (int lvl = -1;; ++lvl) {
-        const int64_t f = fx_eval(tm, node, sc);
+        const int64_t f = fx_eval<RMAX, TW, FR>(tm, node, sc);
         if (lvl < 0) {
             if (f <= 16 * E) return false;
             m = f;
@@ -297,12 +305,14 @@ __device__ __forceinline__ bool fx_descend(FxTeam<RMAX, TW> &tm, const double *_
 // offset inside one block needs no more than FP32: a boundary is that close
 // for about one sample in 10^3.
 // Error: q_r = sum_a u_ra x_a is off by at most gamma A_r, A_r = sum |u_ra x_a|,
-// gamma = 2^-20 (x cut to 24 bits, u rounded, at most nine roundings of the
-// sum); sum_r A_r^2 <= R sum_ra (u_ra x_a)^2 = R S, so the sum of the q_r^2 is
+// gamma = 2^-20 (x and u cut to 24 bits, at most nine roundings of the sum;
+// u is scaled by a power of two above the root of the tree's largest diagonal
+// entry, so no |u| exceeds 2 and what underflows is far below the total that
+// is asked for); sum_r A_r^2 <= R sum_ra (u_ra x_a)^2 = R S, so the sum of the q_r^2 is
 // off by at most 2 gamma sqrt(total R S) + gamma^2 R S.
 template <int RMAX, int TW>
 __device__ __forceinline__ bool fx_leaf_scan(FxTeam<RMAX, TW> &tm, const double *__restrict__ U, int R, const DGeom &g,
-                                             const FxLeaf &lf, int64_t &row) {
+                                             const FxLeaf &lf, int eg, int64_t &row) {
     constexpr int XPL = Shape<RMAX>::XPL, FQ = Shape<RMAX>::FQ;
     constexpr int K = 16;
     const int lane = tm.tid & 31, warp = tm.tid >> 5;
@@ -313,6 +323,7 @@ __device__ __forceinline__ bool fx_leaf_scan(FxTeam<RMAX, TW> &tm, const double 
 #pragma unroll
     for (int q = 0; q < XPL; ++q) x[q] = lane + 32 * q < R ? tm.xs[lane + 32 * q].x : 0.0f;
     float sq = 0.0f;
+    const int uadj = -((eg + 1023) / 2 + 1 - 127) * (1 << 20);
 #pragma unroll 1
     for (int r0 = K * warp; r0 < F; r0 += K * TW) {
         float v[K];
@@ -320,11 +331,12 @@ __device__ __forceinline__ bool fx_leaf_scan(FxTeam<RMAX, TW> &tm, const double 
         for (int rr = 0; rr < K; ++rr) {
             v[rr] = 0.0f;
             if (r0 + rr < rows) {
-                const double *u = U + (row0 + r0 + rr) * (int64_t)R;
+                const uint2 *u = reinterpret_cast<const uint2 *>(U + (row0 + r0 + rr) * (int64_t)R);
 #pragma unroll
                 for (int q = 0; q < XPL; ++q)
                     if (lane + 32 * q < R) {
-                        const float p = d2f_rn(__ldg(u + lane + 32 * q)) * x[q];
+                        const uint2 w = __ldg(u + lane + 32 * q);
+                        const float p = fx_upper(w.y, w.x, uadj) * x[q];
                         v[rr] += p;
                         sq = fmaf(p, p, sq);
                     }

@@ -4,8 +4,15 @@
 // those are certain, from the FP64 code of descent.cuh where they are not.
 // The FP64 work left per sample is h o W[u], the update of h and the weight.
 //
+// Measured (one GB300; FP64 forms before, this kernel now): N = 3, I = 2^22,
+// R = 32, J = 50,000, one mode excluded 6.25 -> 2.24 ms; N = 4, I = 1000,
+// R = 8, J = 10,000 with copies to the host 0.93 -> 0.20 ms.  It is bound by
+// the integer pipe (cutting the FP64 values, 46% of its peak) and the latency
+// of the node reads.
+//
 // One warp per sample up to R = 64 (at R = 32 a query's outer product takes
-// 4.2 KB of shared memory and 24 warps run per SM); above, a team of four
+// 4.2 KB of shared memory; 32 warps of 64 registers per SM measured 3% faster
+// than 24 of 80); above, a team of four
 // warps shares one sample, since a query of R = 100 takes 40 KB and one warp
 // per sample would leave five warps on an SM.
 #include <algorithm>
@@ -19,8 +26,14 @@ struct FxShape {
     static constexpr int TW = RMAX <= 64 ? 1 : 4;          // warps per sample
     static constexpr int TEAMS = RMAX <= 64 ? 4 : 1;       // samples per block
     static constexpr int THREADS = 32 * TW * TEAMS;
-    static constexpr int MINB = RMAX <= 32 ? 6 : (RMAX <= 64 ? 3 : 4);  // blocks per SM
+    static constexpr int MINB = RMAX <= 32 ? 8 : (RMAX <= 64 ? 3 : 4);  // blocks per SM
 };
+
+// Block header: exponents of the roots, a redo's result, then the pair table.
+constexpr int kFxHead = 2 * FTL_MAX_MODES * (int)sizeof(int) + 16;
+__host__ __device__ inline size_t fx_head(int R) {
+    return kFxHead + ((size_t)(node_stride(R, 8) / 2) * sizeof(uint16_t) + 15) / 16 * 16;
+}
 
 // Shared memory of one team, and where its parts lie.
 template <int RMAX>
@@ -45,16 +58,21 @@ struct FxSmem {
 };
 
 // xx of the FP64 form into the team's slot (QForm<., double>::setup's values).
-__device__ __forceinline__ void fx_fill64(double *s, const double *x, int R, int P, int S, int lane) {
-    for (int e = lane; e < S; e += 32) {
-        double v = 0.0;
-        if (e < P) {
-            int a, b;
-            pair_of(e, R, a, b);
-            v = x[a] * x[b];
-            if (a != b) v += v;
+__device__ __forceinline__ void fx_fill64(double *s, const double *x, const uint16_t *pairs, int R, int P, int S,
+                                          int lane) {
+    for (int v = lane; 2 * v < S; v += 32) {
+        const unsigned pr = pairs[v];
+        int a = (int)(pr >> 8), b = (int)(pr & 0xffu);
+        double o[2] = {0.0, 0.0};
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+            if (2 * v + w < P) {
+                o[w] = x[a] * x[b];
+                if (a != b) o[w] += o[w];
+            }
+            if (++b == R) b = ++a;
         }
-        s[e] = v;
+        *reinterpret_cast<double2 *>(s + 2 * v) = make_double2(o[0], o[1]);
     }
     __syncwarp();
 }
@@ -64,12 +82,13 @@ __device__ __forceinline__ void fx_fill64(double *s, const double *x, int R, int
 // else the leaf index.
 template <int RMAX>
 __device__ __noinline__ int64_t fx_redo(const DrawParams &p, const double *G, const DGeom &g, const double *U,
-                                        double *slot, const double *xd, double u, bool with_rows, int lane) {
+                                        double *slot, const double *xd, const uint16_t *pairs, double u,
+                                        bool with_rows, int lane) {
     QForm<RMAX, double> qf;
     qf.P = p.P;
     qf.S = p.S;
     qf.s = slot;
-    fx_fill64(slot, xd, p.R, p.P, p.S, lane);
+    fx_fill64(slot, xd, pairs, p.R, p.P, p.S, lane);
     double frac;
     const int64_t c = descend<RMAX>(G, p.S, g, u, qf, lane, frac);
     if (!with_rows || g.F <= 1) return leaf_index(g, c);
@@ -77,7 +96,7 @@ __device__ __noinline__ int64_t fx_redo(const DrawParams &p, const double *G, co
     return leaf_scan<RMAX, double, double>(U, p.R, g, c, frac, lane_query<RMAX, double>(xd, p.R, lane), lane, empty);
 }
 
-template <int RMAX>
+template <int RMAX, int FR>
 __global__ void __launch_bounds__(FxShape<RMAX>::THREADS, FxShape<RMAX>::MINB) krp_draw_fx_kernel(DrawParams p) {
     using Sh = FxShape<RMAX>;
     constexpr int TW = Sh::TW, TEAMS = Sh::TEAMS;
@@ -90,17 +109,24 @@ __global__ void __launch_bounds__(FxShape<RMAX>::THREADS, FxShape<RMAX>::MINB) k
     int *eg = (int *)smem_raw;  // largest diagonal exponent of the roots: [eigen trees, Gram trees][N]
     int64_t *answer = (int64_t *)(smem_raw + 2 * FTL_MAX_MODES * sizeof(int));  // TW > 1: a redo's result
     const FxSmem<RMAX> lay(R);
-    unsigned char *base = smem_raw + 2 * FTL_MAX_MODES * sizeof(int) + 16 + (threadIdx.x / (32 * TW)) * lay.team;
+    uint16_t *pairs = (uint16_t *)(smem_raw + kFxHead);
+    unsigned char *base = smem_raw + fx_head(R) + (threadIdx.x / (32 * TW)) * lay.team;
     Team tm;
     tm.slot = (float4 *)(base + lay.slot);
     tm.xd = (double *)(base + lay.xd);
     tm.xs = (float2 *)(base + lay.xs);
     tm.qrow = (float *)(base + lay.qrow);
     tm.red = (int2 *)(base + lay.red);
+    tm.pairs = pairs;
     tm.tid = threadIdx.x % (32 * TW);
     tm.nvec = p.S / 2;
     tm.fr = tm.nvec / (32 * TW);
     tm.flip = 0;
+    for (int v = threadIdx.x; v < tm.nvec; v += Sh::THREADS) {
+        int a, b;
+        pair_of(min(2 * v, p.P - 1), R, a, b);
+        pairs[v] = (uint16_t)((a << 8) | b);
+    }
     for (int k = threadIdx.x >> 5; k < 2 * N; k += TW * TEAMS) {
         const int mode = k % N;
         unsigned e = 0;
@@ -157,12 +183,12 @@ __global__ void __launch_bounds__(FxShape<RMAX>::THREADS, FxShape<RMAX>::MINB) k
                         lf.m = (int64_t)1 << 53;
                         lf.tol = lf.mtol = 1;
                     } else {
-                        ok = fx_descend(tm, G, p.S, g, Dk, sc, lf);
+                        ok = fx_descend<RMAX, TW, FR>(tm, G, p.S, g, Dk, sc, lf);
                     }
                 }
                 if (ok) {
                     if (phase == 1 && g.F > 1)
-                        ok = fx_leaf_scan(tm, p.U[k], R, g, lf, t);
+                        ok = fx_leaf_scan(tm, p.U[k], R, g, lf, eg[l], t);
                     else
                         t = leaf_index(g, (int64_t)lf.c);
                 }
@@ -170,7 +196,7 @@ __global__ void __launch_bounds__(FxShape<RMAX>::THREADS, FxShape<RMAX>::MINB) k
                     const double u = get_draw(p, (int64_t)l * p.J + i);
                     Team::sync();
                     if (TW == 1 || tm.tid < 32) {
-                        t = fx_redo<RMAX>(p, G, g, p.U[k], (double *)tm.slot, tm.xd, u, phase == 1, lane);
+                        t = fx_redo<RMAX>(p, G, g, p.U[k], (double *)tm.slot, tm.xd, tm.pairs, u, phase == 1, lane);
                         if (TW > 1 && lane == 0) *answer = t;
                     }
                     Team::sync();
@@ -206,7 +232,7 @@ __global__ void __launch_bounds__(FxShape<RMAX>::THREADS, FxShape<RMAX>::MINB) k
                 qf.P = p.P;
                 qf.S = p.S;
                 qf.s = (double *)tm.slot;
-                fx_fill64(qf.s, tm.xd, R, p.P, p.S, lane);
+                fx_fill64(qf.s, tm.xd, tm.pairs, R, p.P, p.S, lane);
                 const double lev = qf.eval(p.M + cm_pinv64_offset(N, R), lane);
                 if (lane == 0) p.weights[i] = (double)R / (lev * (double)p.J);
             }
@@ -220,28 +246,37 @@ __global__ void __launch_bounds__(FxShape<RMAX>::THREADS, FxShape<RMAX>::MINB) k
     }
 }
 
-template <int RMAX>
+template <int RMAX, int FR>
 static int launch_fx(const DrawParams &p, cudaStream_t st) {
     using Sh = FxShape<RMAX>;
-    const size_t smem = 2 * FTL_MAX_MODES * sizeof(int) + 16 + Sh::TEAMS * FxSmem<RMAX>(p.R).team;
-    int rc = ensure_smem((const void *)krp_draw_fx_kernel<RMAX>, smem, "krp_draw_fx_kernel");
+    const auto kernel = krp_draw_fx_kernel<RMAX, FR>;
+    const size_t smem = fx_head(p.R) + Sh::TEAMS * FxSmem<RMAX>(p.R).team;
+    int rc = ensure_smem((const void *)kernel, smem, "krp_draw_fx_kernel");
     if (rc) return rc;
     // one wave of resident blocks, each looping over samples
     int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, krp_draw_fx_kernel<RMAX>, Sh::THREADS, smem) !=
-            cudaSuccess ||
-        occ < 1)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, Sh::THREADS, smem) != cudaSuccess || occ < 1)
         occ = 1;
     const int64_t need = (p.J + Sh::TEAMS - 1) / Sh::TEAMS;
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)num_sms() * occ));
-    krp_draw_fx_kernel<RMAX><<<blocks, Sh::THREADS, smem, st>>>(p);
+    kernel<<<blocks, Sh::THREADS, smem, st>>>(p);
     return check_launch("krp_draw_fx_kernel");
 }
 
 int launch_draw_fx(const DrawParams &p, cudaStream_t st) {
-    if (p.R <= 32) return launch_fx<32>(p, st);
-    if (p.R <= 64) return launch_fx<64>(p, st);
-    return launch_fx<128>(p, st);
+    if (p.R > 64) return launch_fx<128, -1>(p, st);
+    if (p.R > 32) return launch_fx<64, -1>(p, st);
+    switch (p.S / 64) {  // full rows of 32 two-entry vectors in a node
+        case 0: return launch_fx<32, 0>(p, st);
+        case 1: return launch_fx<32, 1>(p, st);
+        case 2: return launch_fx<32, 2>(p, st);
+        case 3: return launch_fx<32, 3>(p, st);
+        case 4: return launch_fx<32, 4>(p, st);
+        case 5: return launch_fx<32, 5>(p, st);
+        case 6: return launch_fx<32, 6>(p, st);
+        case 7: return launch_fx<32, 7>(p, st);
+        default: return launch_fx<32, 8>(p, st);
+    }
 }
 
 }  // namespace ftl
