@@ -155,8 +155,9 @@ class ALS:
         N, R = lr.N, lr.R
         j = int(j)
         st = D.stream_ptr(self.device)
-        G = [factor_gram(u, self._ws, st) for u in lr.U_dev]
         gram = torch.empty((R, R), dtype=torch.float64, device=self.device)
+        # mode j's own Gram does not enter the product (its slot is not read)
+        G = [gram if k == j else factor_gram(u, self._ws, st) for k, u in enumerate(lr.U_dev)]
         _lib.call("ftl_gram_hadamard", _ptrs(G), N, R, j, None, None, gram.data_ptr(), None, st)
         pinv = torch.empty((R, R), dtype=torch.float64, device=self.device)
         vscr = torch.empty((R, R), dtype=torch.float64, device=self.device)

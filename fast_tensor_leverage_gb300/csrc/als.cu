@@ -780,63 +780,88 @@ __device__ __forceinline__ void fiber_normals(uint64_t seed, uint32_t mode, uint
     z1 = r * sn;
 }
 
+// (double)x for a finite x that is zero or normal, by integer operations: the
+// conversion runs on the FP64 pipe, where a warp instruction takes 64 cycles.
+__device__ __forceinline__ double f2d_exact(float x) {
+    const uint32_t b = __float_as_uint(x), a = b & 0x7fffffffu;
+    const uint32_t hi = (b & 0x80000000u) | (a ? (a >> 3) + 0x38000000u : 0u);
+    return __hiloint2double((int)hi, (int)(b << 29));
+}
+
 // out[idx_j(z), :] += val(z) * g(fiber(z)) over the nonzeros sorted by their
 // mode-j index (SortIdxLookup::execute_rrf, sort_lookup.hpp:262-353: one
-// Gaussian R-vector per fiber).  Chunks of MTT_CHUNK nonzeros per warp, lane
-// l owns column pairs l, l + 32, ...; per-row accumulation, one atomic add
-// per column when the row changes.
+// Gaussian R-vector per fiber).  A chunk of RRF_CHUNK nonzeros per warp, cut
+// into one run per slot of a warp: a slot is as many lanes as the vector has
+// column pairs (PPL = 1: R <= 64; one pair per lane), so that R = 25 uses 26
+// of 32 lanes instead of 13.  Per-row accumulation, one atomic add per column
+// when the row changes.  Bound by the generator's integer and FP32 work and
+// by two FP64 multiply-adds per lane and nonzero: three modes of 6.3e6
+// nonzeros at R = 25 took 4.93 ms with one slot and FP64 conversions.
 constexpr int RRF_CHUNK = 512;
 
-__global__ void rrf_rows_kernel(const int32_t *__restrict__ rrows, const uint64_t *__restrict__ rkeys,
-                                const double *__restrict__ rvals, int64_t nnz, int R, uint64_t seed, uint32_t mode,
-                                double *__restrict__ out) {
+template <int PPL>
+__global__ void __launch_bounds__(256) rrf_rows_kernel(const int32_t *__restrict__ rrows,
+                                                       const uint64_t *__restrict__ rkeys,
+                                                       const double *__restrict__ rvals, int64_t nnz, int R,
+                                                       uint64_t seed, uint32_t mode, double *__restrict__ out) {
     const int lane = threadIdx.x & 31;
     const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    constexpr int PPL = (FTL_MAX_RANK / 2 + 31) / 32;  // column pairs per lane
     const int npairs = (R + 1) / 2;
+    const int slots = PPL == 1 ? 32 / npairs : 1;
+    const int slot = PPL == 1 ? lane / npairs : 0;
+    const int pair = PPL == 1 ? lane - slot * npairs : lane;
+    const int run = (RRF_CHUNK + slots - 1) / slots;
     const int64_t nchunks = (nnz + RRF_CHUNK - 1) / RRF_CHUNK;
+    if (slot >= slots) return;  // no warp-wide operation below
     for (int64_t ch = gw; ch < nchunks; ch += nw) {
-        const int64_t z0 = ch * RRF_CHUNK, z1 = min(nnz, z0 + RRF_CHUNK);
+        const int64_t end = min(nnz, (ch + 1) * RRF_CHUNK);
+        const int64_t z0 = ch * RRF_CHUNK + (int64_t)slot * run, z1 = min(end, z0 + run);
         double acc[2 * PPL];
 #pragma unroll
         for (int c = 0; c < 2 * PPL; ++c) acc[c] = 0.0;
-        int32_t cur = -1;
-        for (int64_t z = z0; z < z1; ++z) {
-            const int32_t row = rrows[z];
-            const uint64_t key = rkeys[z];
-            const double v = rvals[z];
-            if (row != cur) {
-                if (cur >= 0) {
+        int32_t cur = -1, nrow = -1;
+        uint64_t nkey = 0;
+        double nval = 0.0;
+        auto flush = [&] {
 #pragma unroll
-                    for (int q = 0; q < PPL; ++q) {
-                        const int pp = lane + 32 * q;
-                        if (2 * pp < R) atomicAdd(out + (int64_t)cur * R + 2 * pp, acc[2 * q]);
-                        if (2 * pp + 1 < R) atomicAdd(out + (int64_t)cur * R + 2 * pp + 1, acc[2 * q + 1]);
-                        acc[2 * q] = acc[2 * q + 1] = 0.0;
-                    }
-                }
+            for (int q = 0; q < PPL; ++q) {
+                const int pp = pair + 32 * q;
+                if (2 * pp < R) atomicAdd(out + (int64_t)cur * R + 2 * pp, acc[2 * q]);
+                if (2 * pp + 1 < R) atomicAdd(out + (int64_t)cur * R + 2 * pp + 1, acc[2 * q + 1]);
+                acc[2 * q] = acc[2 * q + 1] = 0.0;
+            }
+        };
+        if (z0 < z1) {
+            nrow = rrows[z0];
+            nkey = rkeys[z0];
+            nval = rvals[z0];
+        }
+        for (int64_t z = z0; z < z1; ++z) {
+            const int32_t row = nrow;
+            const uint64_t key = nkey;
+            const double v = nval;
+            if (z + 1 < z1) {  // the next nonzero's loads overlap this one's generator
+                nrow = rrows[z + 1];
+                nkey = rkeys[z + 1];
+                nval = rvals[z + 1];
+            }
+            if (row != cur) {
+                if (cur >= 0) flush();
                 cur = row;
             }
 #pragma unroll
             for (int q = 0; q < PPL; ++q) {
-                const int pp = lane + 32 * q;
+                const int pp = pair + 32 * q;
                 if (pp < npairs) {
                     float g0, g1;
                     fiber_normals(seed, mode, key, (uint32_t)pp, g0, g1);
-                    acc[2 * q] = fma(v, (double)g0, acc[2 * q]);
-                    acc[2 * q + 1] = fma(v, (double)g1, acc[2 * q + 1]);
+                    acc[2 * q] = fma(v, f2d_exact(g0), acc[2 * q]);
+                    acc[2 * q + 1] = fma(v, f2d_exact(g1), acc[2 * q + 1]);
                 }
             }
         }
-        if (cur >= 0) {
-#pragma unroll
-            for (int q = 0; q < PPL; ++q) {
-                const int pp = lane + 32 * q;
-                if (2 * pp < R) atomicAdd(out + (int64_t)cur * R + 2 * pp, acc[2 * q]);
-                if (2 * pp + 1 < R) atomicAdd(out + (int64_t)cur * R + 2 * pp + 1, acc[2 * q + 1]);
-            }
-        }
+        if (cur >= 0) flush();
     }
 }
 
@@ -1048,6 +1073,135 @@ __global__ void exact_mttkrp_kernel(const uint32_t *__restrict__ idx, const doub
             atomicAdd(o + r, v * p);
         }
     }
+}
+
+// The same sum over the nonzeros sorted by their mode-j index, each with its
+// row and fiber key: a group of GW lanes (the columns; GW = 8, 16 or 32, CPL
+// columns per lane) walks a contiguous run, every lane reads one nonzero of
+// the next GW and takes the other modes' indices out of its key (the key's
+// mixed-radix digits), and the group applies them one after the other to a
+// per-row accumulator, flushed with one atomic add per column when the row
+// changes -- instead of one per nonzero and column.  Bound by the FP64 pipe:
+// N - 1 multiply(-add)s per nonzero and group of lanes.  6.3e6 nonzeros of 3
+// modes at R = 25: 6.1 ms with an atomic per nonzero and column, 1.2 ms here.
+constexpr int EXM_RUN = 256;  // nonzeros per group and visit
+
+struct KeyDigits {
+    int n;  // modes other than j, last first
+    uint64_t size[FTL_MAX_MODES];
+    const double *U[FTL_MAX_MODES];
+};
+
+template <int GW, int CPL, int NK>
+__global__ void __launch_bounds__(256) exact_mttkrp_rows_kernel(const int32_t *__restrict__ rrows,
+                                                                const uint64_t *__restrict__ rkeys,
+                                                                const double *__restrict__ rvals, int64_t nnz,
+                                                                KeyDigits kd, int R, double *__restrict__ out) {
+    constexpr int NG = 32 / GW, G = 4;
+    const int lane = threadIdx.x & 31, gl = lane % GW;
+    const int64_t gid = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * NG + lane / GW;
+    const int64_t ngroups = (((int64_t)gridDim.x * blockDim.x) >> 5) * NG;
+    const int64_t nruns = (nnz + EXM_RUN - 1) / EXM_RUN;
+    const int64_t visits = (nruns + ngroups - 1) / ngroups;  // the same for every group: shuffles below
+    for (int64_t vis = 0; vis < visits; ++vis) {
+        const int64_t z0 = (vis * ngroups + gid) * EXM_RUN, z1 = min(nnz, z0 + EXM_RUN);
+        double acc[CPL];
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) acc[c] = 0.0;
+        int32_t cur = -1;
+        auto flush = [&] {
+#pragma unroll
+            for (int c = 0; c < CPL; ++c) {
+                const int col = gl + GW * c;
+                if (col < R) atomicAdd(out + (int64_t)cur * R + col, acc[c]);
+                acc[c] = 0.0;
+            }
+        };
+        for (int b = 0; b < EXM_RUN; b += GW) {
+            const int64_t z = z0 + b + gl;
+            int32_t row = -1;
+            double val = 0.0;
+            uint32_t id[NK];
+#pragma unroll
+            for (int k = 0; k < NK; ++k) id[k] = 0;
+            if (z < z1) {
+                row = rrows[z];
+                val = rvals[z];
+                uint64_t key = rkeys[z];
+#pragma unroll
+                for (int k = 0; k < NK; ++k) {
+                    if (k < kd.n) {
+                        if (k + 1 < kd.n) {
+                            const uint64_t q = key / kd.size[k];
+                            id[k] = (uint32_t)(key - q * kd.size[k]);
+                            key = q;
+                        } else {
+                            id[k] = (uint32_t)key;
+                        }
+                    }
+                }
+            }
+#pragma unroll 1
+            for (int g0 = 0; g0 < GW; g0 += G) {
+                int32_t hr[G];
+                double pr[G][CPL], u0[G][CPL];  // value times the other factors' rows, and mode kd.U[0]'s row
+#pragma unroll
+                for (int g = 0; g < G; ++g) {
+                    hr[g] = __shfl_sync(0xffffffffu, row, g0 + g, GW);
+                    const double v = __shfl_sync(0xffffffffu, val, g0 + g, GW);
+#pragma unroll
+                    for (int c = 0; c < CPL; ++c) {
+                        pr[g][c] = v;
+                        u0[g][c] = 1.0;
+                    }
+#pragma unroll
+                    for (int k = 0; k < NK; ++k) {
+                        if (k < kd.n) {
+                            const uint32_t i = __shfl_sync(0xffffffffu, id[k], g0 + g, GW);
+                            const double *u = kd.U[k] + (int64_t)i * R;
+#pragma unroll
+                            for (int c = 0; c < CPL; ++c) {
+                                const int col = gl + GW * c;
+                                if (hr[g] >= 0 && col < R) {
+                                    if (k == 0) u0[g][c] = u[col];
+                                    else pr[g][c] *= u[col];
+                                }
+                            }
+                        }
+                    }
+                }
+#pragma unroll
+                for (int g = 0; g < G; ++g) {
+                    if (hr[g] >= 0) {
+                        if (hr[g] != cur) {
+                            if (cur >= 0) flush();
+                            cur = hr[g];
+                        }
+#pragma unroll
+                        for (int c = 0; c < CPL; ++c) acc[c] = fma(pr[g][c], u0[g][c], acc[c]);
+                    }
+                }
+                __syncwarp();
+            }
+        }
+        if (cur >= 0) flush();
+        __syncwarp();
+    }
+}
+
+template <int GW, int CPL>
+static void launch_exact_rows(const int32_t *rrows, const uint64_t *rkeys, const double *rvals, int64_t nnz,
+                              const KeyDigits &kd, int R, double *out, cudaStream_t st) {
+    const int64_t per_block = 8 * (32 / GW) * (int64_t)EXM_RUN;
+    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((nnz + per_block - 1) / per_block,
+                                                                   (int64_t)num_sms() * 32));
+    if (kd.n <= 2)
+        exact_mttkrp_rows_kernel<GW, CPL, 2><<<blocks, 256, 0, st>>>(rrows, rkeys, rvals, nnz, kd, R, out);
+    else if (kd.n <= 3)
+        exact_mttkrp_rows_kernel<GW, CPL, 3><<<blocks, 256, 0, st>>>(rrows, rkeys, rvals, nnz, kd, R, out);
+    else
+        exact_mttkrp_rows_kernel<GW, CPL, FTL_MAX_MODES - 1>
+            <<<blocks, 256, 0, st>>>(rrows, rkeys, rvals, nnz, kd, R, out);
 }
 
 struct GramPtrs {
@@ -1396,6 +1550,42 @@ extern "C" int ftl_sparse_exact_mttkrp(const uint32_t *idx, const double *vals, 
     return check_launch("exact_mttkrp_kernel");
 }
 
+extern "C" int ftl_sparse_exact_mttkrp_rows(const int32_t *row_idx, const uint64_t *row_keys, const double *row_vals,
+                                            int64_t nnz, int N, const int64_t *dims, int j,
+                                            const double *const *U_dev, int R, double *out, int64_t I_j,
+                                            void *stream) {
+    FTL_CHECK_ARG(row_idx && row_keys && row_vals && dims && U_dev && out,
+                  "ftl_sparse_exact_mttkrp_rows: null pointer");
+    FTL_CHECK_ARG(N >= 1 && N <= FTL_MAX_MODES && j >= 0 && j < N && R >= 1 && R <= FTL_MAX_RANK && I_j >= 1 &&
+                      nnz >= 0,
+                  "ftl_sparse_exact_mttkrp_rows: bad shape");
+    KeyDigits kd;
+    kd.n = 0;
+    for (int k = N - 1; k >= 0; --k) {
+        FTL_CHECK_ARG(dims[k] >= 1, "ftl_sparse_exact_mttkrp_rows: dims[%d]=%lld", k, (long long)dims[k]);
+        if (k == j) continue;
+        FTL_CHECK_ARG(U_dev[k], "ftl_sparse_exact_mttkrp_rows: factor %d is NULL", k);
+        kd.U[kd.n] = U_dev[k];
+        kd.size[kd.n++] = (uint64_t)dims[k];
+    }
+    cudaStream_t st = (cudaStream_t)stream;
+    cudaError_t err = cudaMemsetAsync(out, 0, (size_t)I_j * R * sizeof(double), st);
+    if (err != cudaSuccess)
+        return fail(FTL_E_CUDA, "ftl_sparse_exact_mttkrp_rows: memset: %s", cudaGetErrorString(err));
+    if (nnz == 0) return FTL_OK;
+    if (R <= 8)
+        launch_exact_rows<8, 1>(row_idx, row_keys, row_vals, nnz, kd, R, out, st);
+    else if (R <= 16)
+        launch_exact_rows<16, 1>(row_idx, row_keys, row_vals, nnz, kd, R, out, st);
+    else if (R <= 32)
+        launch_exact_rows<32, 1>(row_idx, row_keys, row_vals, nnz, kd, R, out, st);
+    else if (R <= 64)
+        launch_exact_rows<32, 2>(row_idx, row_keys, row_vals, nnz, kd, R, out, st);
+    else
+        launch_exact_rows<32, 4>(row_idx, row_keys, row_vals, nnz, kd, R, out, st);
+    return check_launch("exact_mttkrp_rows_kernel");
+}
+
 extern "C" int ftl_sparse_rrf(const int32_t *row_idx, const uint64_t *row_keys, const double *row_vals, int64_t nnz,
                               int R, uint64_t seed, uint32_t mode, double *out, int64_t I_j, void *stream) {
     FTL_CHECK_ARG(row_idx && row_keys && row_vals && out, "ftl_sparse_rrf: null pointer");
@@ -1407,6 +1597,9 @@ extern "C" int ftl_sparse_rrf(const int32_t *row_idx, const uint64_t *row_keys, 
     if (nnz == 0) return FTL_OK;
     const int64_t nchunks = (nnz + RRF_CHUNK - 1) / RRF_CHUNK;
     int blocks = (int)std::min<int64_t>((nchunks * 32 + 255) / 256, (int64_t)num_sms() * 32);
-    rrf_rows_kernel<<<std::max(blocks, 1), 256, 0, st>>>(row_idx, row_keys, row_vals, nnz, R, seed, mode, out);
+    if (R <= 64)
+        rrf_rows_kernel<1><<<std::max(blocks, 1), 256, 0, st>>>(row_idx, row_keys, row_vals, nnz, R, seed, mode, out);
+    else
+        rrf_rows_kernel<2><<<std::max(blocks, 1), 256, 0, st>>>(row_idx, row_keys, row_vals, nnz, R, seed, mode, out);
     return check_launch("rrf_rows_kernel");
 }

@@ -559,8 +559,9 @@ class SparseTensor:
 
     def _exact_mttkrp_dev(self, U_L, j: int, out, out_rows, stream) -> None:
         R = int(U_L[0].shape[1])
-        _lib.call("ftl_sparse_exact_mttkrp", self.idx_dev.data_ptr(), self.vals_dev.data_ptr(), self.nnz, self.N, j,
-                  _ptrs(U_L), R, out, out_rows, stream)
+        rrows, rkeys, rvals = self.rows[j]
+        _lib.call("ftl_sparse_exact_mttkrp_rows", rrows.data_ptr(), rkeys.data_ptr(), rvals.data_ptr(), self.nnz,
+                  self.N, self._dims_c, j, _ptrs(U_L), R, out, out_rows, stream)
 
     def execute_rrf(self, lr: "LowRankTensor", seed: int | None = None) -> None:
         """Randomized range-finder initialisation of `lr` (SparseTensor::

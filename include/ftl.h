@@ -388,6 +388,15 @@ int ftl_sparse_exact_mttkrp(const uint32_t *idx_dev, const double *vals_dev, int
                             int j, const double *const *U_dev, int R, double *out_dev,
                             int64_t I_j, void *stream);
 
+/* The same sum over the nonzeros sorted by their mode-j index (row_idx, with
+ * fiber keys row_keys over tensor sizes dims, as ftl_fiber_keys forms them, and
+ * values row_vals): one atomic add per column and row segment instead of one
+ * per column and nonzero. */
+int ftl_sparse_exact_mttkrp_rows(const int32_t *row_idx, const uint64_t *row_keys, const double *row_vals,
+                                 int64_t nnz, int N, const int64_t *dims, int j,
+                                 const double *const *U_dev, int R, double *out, int64_t I_j,
+                                 void *stream);
+
 /* Randomized range finder of mode j (SortIdxLookup::execute_rrf,
  * cpp_ext/sort_lookup.hpp:262-353): out (I_j x R, zeroed first) = X_(j) Omega,
  * Omega holding one N(0,1) R-vector per fiber (modes != j).  Inputs are the
