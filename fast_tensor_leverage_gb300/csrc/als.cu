@@ -382,7 +382,7 @@ __global__ void pinv_square_kernel(const double *__restrict__ M, int R, int targ
         A[e] = a <= b ? M[e] : M[b * R + a];
     }
     __syncthreads();
-    jacobi_eigen<double>(A, V, R, cs, pq, flag);
+    jacobi64<false>(OwnMat{A}, OwnMat{V}, R, cs, pq, flag, 0, 1);
     sort_ascending<double>(A, R, order);
     for (int e = tid; e < RR; e += nth) {
         int a = e / R, b = e - a * R;

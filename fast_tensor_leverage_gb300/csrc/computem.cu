@@ -170,7 +170,7 @@ __global__ void computem_pinv_kernel(CMParams p) {
     if (!chol) {
     for (int e = tid; e < RR; e += nth) A[e] = p.M[e];
     __syncthreads();
-    jacobi_eigen<double>(A, V, R, cs, pq, flag);
+    jacobi64<false>(OwnMat{A}, OwnMat{V}, R, cs, pq, flag, 0, 1);
     sort_ascending<double>(A, R, order);
     // W = M[N]: row (R-1-r) = v_r / sqrt(lambda_r) for lambda_r > 1e-8, else 0,
     // r the ascending rank (column R-1-r of the reference's V Lambda^{-1/2}).
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(FTL_CM_THREADS) computem_eig_kernel(CMParams p
             // the PSD matrix by one warp (one-sided Jacobi in registers)
             if (tid < 32) warp_jacobi_psd32(A32, R, k, W, p.lambda + (size_t)offset * R, tid);
         } else {
-            jacobi_eigen<float>(A32, V32, R, cs32, pq32, flag32);
+            jacobi_eigen32(A32, V32, R, cs32, pq32, flag32);
             sort_ascending<float>(A32, R, order32);
             const double wsc = ldexp(1.0, -k / 2), lsc = ldexp(1.0, -k);
             for (int e = tid; e < RR; e += nth) {
@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(FTL_CM_THREADS) computem_eig_kernel(CMParams p
     } else if (offset < N) {
         for (int e = tid; e < RR; e += nth) A[e] = W[e];
         __syncthreads();
-        jacobi_eigen<double>(A, V, R, cs, pq, flag);
+        jacobi64<false>(OwnMat{A}, OwnMat{V}, R, cs, pq, flag, 0, 1);
         sort_ascending<double>(A, R, order);
         // row r = sqrt(lambda_r) v_r, ascending (negative rounding noise -> 0)
         for (int e = tid; e < RR; e += nth) {
@@ -411,6 +411,141 @@ __global__ void __launch_bounds__(FTL_CM_THREADS) computem_eig_kernel(CMParams p
     for (int e = tid; e < (2 * R - 1) * S; e += nth) G[e] = G[e] * root[e % S];
 }
 
+// ------------------------------------------------- FP64, R > 32: clusters
+//
+// One CTA has an SM's FP64 pipe: two lanes per cycle.  A Jacobi round at R =
+// 100 is 40,000 FP64 lane operations and the two eigensolves took 19.2 and
+// 19.8 ms.  A cluster of eight CTAs shares one matrix in L2 (A in its M slot,
+// V in its scratch slot); every other step is split over the cluster's threads
+// so that an entry stays with one thread and needs no exchange.
+constexpr int kCmCluster = 8;
+constexpr int kCmClThreads = 512;
+
+struct CMClShared {
+    double cs[FTL_MAX_RANK + 2], lam[FTL_MAX_RANK];
+    int pq[FTL_MAX_RANK + 2], order[FTL_MAX_RANK], flag;
+};
+
+// Eigenvalues from A's diagonal and their ascending order (sort_ascending's
+// rule), in every CTA.
+__device__ __forceinline__ void cl_sort(CMClShared &sm, const ClusterMat A, int R) {
+    for (int v = threadIdx.x; v < R; v += blockDim.x) sm.lam[v] = A.ld(v * R + v);
+    __syncthreads();
+    for (int v = threadIdx.x; v < R; v += blockDim.x) {
+        double lv = sm.lam[v];
+        if (lv != lv) lv = INFINITY;
+        int rank = 0;
+        for (int u = 0; u < R; ++u) {
+            double lu = sm.lam[u];
+            if (lu != lu) lu = INFINITY;
+            if (lu < lv || (lu == lv && u < v)) ++rank;
+        }
+        sm.order[rank] = v;
+    }
+    __syncthreads();
+}
+
+__global__ void __cluster_dims__(kCmCluster, 1, 1) __launch_bounds__(kCmClThreads)
+    computem_pinv_cl_kernel(CMParams p) {
+    __shared__ CMClShared sm;
+    const int R = p.R, RR = R * R, N = p.N, rk = blockIdx.x;
+    const int first = rk * kCmClThreads + threadIdx.x, stride = kCmCluster * kCmClThreads;
+    // suffix Hadamard products, entry by entry
+    for (int e = first; e < RR; e += stride) {
+        const int a = e / R, b = e - a * R;
+        double prev = 1.0;
+        for (int k = N - 1; k >= 0; --k) {
+            if ((uint32_t)k == p.j) continue;
+            prev = root_ab(p, k, a, b) * prev;
+            p.M[(size_t)k * RR + e] = prev;
+        }
+        if (p.j == 0) p.M[e] = prev;
+    }
+    if (first == 0) p.M[cm_status_offset(N, R)] = 0.0;
+    cluster_sync();
+    const ClusterMat A{p.M}, V{p.M + (size_t)(N + 2) * RR};
+    jacobi64<true>(A, V, R, sm.cs, sm.pq, &sm.flag, rk, kCmCluster);
+    cl_sort(sm, A, R);
+    // W = M[N]: row (R-1-r) = v_r / sqrt(lambda_r) for lambda_r > 1e-8, else 0
+    double *W = p.M + (size_t)N * RR;
+    for (int e = first; e < RR; e += stride) {
+        const int row = e / R, a = e - row * R;
+        const int v = sm.order[R - 1 - row];
+        const double lam = sm.lam[v];
+        __stcg(W + e, lam > 1e-8 ? V.ld(a * R + v) / sqrt(lam) : 0.0);
+    }
+    if (rk == 0)
+        for (int r = threadIdx.x; r < R; r += blockDim.x) p.lambda[r] = sm.lam[sm.order[r]];
+    cluster_sync();
+    // pinv = W^T W, summed over W's rows in order; into slot 0, the packed
+    // FP64 and FP32 copies, and the suffix products
+    double *pinv_packed = p.M + cm_pinv64_offset(N, R);
+    for (int e = first; e < RR; e += stride) {
+        const int a = e / R, b = e - a * R;
+        const int lo = min(a, b), hi = max(a, b);
+        double acc = 0.0;
+#pragma unroll 4
+        for (int row = 0; row < R; ++row) acc += __ldcg(W + row * R + lo) * __ldcg(W + row * R + hi);
+        p.M[e] = acc;
+        if (a <= b) {
+            pinv_packed[packed_index(a, b, R)] = acc;
+            p.pinv32[packed_index(a, b, R)] = (float)acc;
+        }
+        for (int k = N - 1; k >= 1; --k)
+            if ((uint32_t)k != p.j) p.M[(size_t)k * RR + e] *= acc;
+    }
+    // zero padding up to the node strides, read by the vectorised forms
+    for (int e = p.P + first; e < node_stride(R, 8); e += stride) pinv_packed[e] = 0.0;
+    for (int e = p.P + first; e < node_stride(R, 4); e += stride) p.pinv32[e] = 0.0f;
+}
+
+__global__ void __cluster_dims__(kCmCluster, 1, 1) __launch_bounds__(kCmClThreads)
+    computem_eig_cl_kernel(CMParams p) {
+    __shared__ CMClShared sm;
+    const int R = p.R, RR = R * R, N = p.N, P = p.P;
+    const int k = blockIdx.x / kCmCluster, rk = blockIdx.x % kCmCluster;
+    if ((uint32_t)k == p.j) return;  // the whole cluster
+    const int first = rk * kCmClThreads + threadIdx.x, stride = kCmCluster * kCmClThreads;
+    const int offset = ((uint32_t)(k + 1) == p.j) ? k + 2 : k + 1;
+    double *W = p.M + (size_t)offset * RR;
+    if (offset < N) {
+        const ClusterMat A{W}, V{p.M + (size_t)(N + 3 + k) * RR};
+        jacobi64<true>(A, V, R, sm.cs, sm.pq, &sm.flag, rk, kCmCluster);
+        cl_sort(sm, A, R);
+        cluster_sync();  // every CTA has the eigenvalues: A's slot can be overwritten
+        // row r = sqrt(lambda_r) v_r, ascending (negative rounding noise -> 0)
+        for (int e = first; e < RR; e += stride) {
+            const int r = e / R, a = e - r * R;
+            const int v = sm.order[r];
+            __stcg(W + e, sqrt(fmax(sm.lam[v], 0.0)) * V.ld(a * R + v));
+        }
+        if (rk == 0)
+            for (int r = threadIdx.x; r < R; r += blockDim.x) p.lambda[(size_t)offset * R + r] = sm.lam[sm.order[r]];
+        cluster_sync();
+    }
+    // Eigen tree over the R rows of W (F = 1): a thread owns node positions and
+    // builds the whole tree at each: leaves, child sums, then o root.
+    const int S = node_stride(R, 8);
+    double *G = (double *)p.eig_G + (size_t)k * (2 * R - 1) * S;
+    const double *root = (const double *)p.root[k];
+    const DGeom g = p.eig;
+    for (int pe = first; pe < S; pe += stride) {
+        int a = 0, rem = pe;
+        while (pe < P && rem >= R - a) {
+            rem -= R - a;
+            ++a;
+        }
+        const int b = a + rem;
+#pragma unroll 4
+        for (int u = 0; u < R; ++u)
+            G[(int)leaf_node(g, u) * S + pe] = pe < P ? __ldcg(W + u * R + a) * __ldcg(W + u * R + b) : 0.0;
+        for (int c = R - 2; c >= 0; --c) G[c * S + pe] = G[(2 * c + 1) * S + pe] + G[(2 * c + 2) * S + pe];
+        const double rt = root[pe];
+#pragma unroll 4
+        for (int c = 0; c < 2 * R - 1; ++c) G[c * S + pe] *= rt;
+    }
+}
+
 #ifndef FTL_CM_THREADS
 #define FTL_CM_THREADS 512
 #endif
@@ -428,6 +563,13 @@ int computem_launch(const ftl_krp_plan *plan, uint32_t j_norm, cudaStream_t st) 
     p.pinv32 = plan->pinv32;
     p.eig_G = plan->eig_G;
     p.eig = to_dgeom(make_geom(plan->R, 1));
+    if (plan->prec == FTL_PREC_FP64 && plan->R > 32) {
+        computem_pinv_cl_kernel<<<kCmCluster, kCmClThreads, 0, st>>>(p);
+        int rc = check_launch("computem_pinv_cl_kernel");
+        if (rc) return rc;
+        computem_eig_cl_kernel<<<kCmCluster * plan->N, kCmClThreads, 0, st>>>(p);
+        return check_launch("computem_eig_cl_kernel");
+    }
     p.v_global = cm_smem_bytes(plan->R, false) > 200 * 1024;
     size_t smem = cm_smem_bytes(plan->R, p.v_global);
     if (smem > 227 * 1024) return fail(FTL_E_UNSUPPORTED, "computeM: R=%d too large", plan->R);

@@ -2,7 +2,7 @@
 // R x R matrices in shared (or global scratch) memory.  Used by computeM and
 // by the ALS pseudo-inverse.
 //
-// jacobi_eigen: cyclic parallel-order (round-robin) two-sided Jacobi; each
+// jacobi_eigen32 (FP32) and jacobi64 (FP64): cyclic parallel-order (round-robin) two-sided Jacobi; each
 // round rotates R/2 disjoint pairs (p, q) with the classical rotation that
 // zeroes a_pq (tau = (a_qq - a_pp) / (2 a_pq), t = sign(tau) / (|tau| +
 // sqrt(1 + tau^2)), c = 1 / sqrt(1 + t^2), s = t c), skipping pairs with
@@ -20,14 +20,15 @@
 
 namespace ftl {
 
-// In-place Jacobi on A (R x R, symmetric, row-major, element type T); V
-// receives the eigenvectors as columns.  All threads of the block must call it.
-template <typename T>
-__device__ void jacobi_eigen(T *A, T *V, int R, T *csbuf, int *pqbuf, int *flag) {
+// In-place Jacobi on A (R x R, symmetric, row-major, FP32); V receives the
+// eigenvectors as columns.  All threads of the block must call it.  (FP64:
+// jacobi64 below.)
+__device__ inline void jacobi_eigen32(float *A, float *V, int R, float *csbuf, int *pqbuf, int *flag) {
+    using T = float;
     const int tid = threadIdx.x, nth = blockDim.x;
     const int n = R + (R & 1);
     const int half = n / 2;
-    const T eps = sizeof(T) == 8 ? T(1.1102230246251565e-16) : T(5.9604645e-08);
+    const T eps = 5.9604645e-08f;
     for (int e = tid; e < R * R; e += nth) V[e] = (e / R == e % R) ? T(1) : T(0);
     __syncthreads();
     for (int sweep = 0; sweep < 40; ++sweep) {
@@ -56,7 +57,7 @@ __device__ void jacobi_eigen(T *A, T *V, int R, T *csbuf, int *pqbuf, int *flag)
                     if (apq != T(0) && fabs(apq) > eps * sqrt(fabs(app * aqq))) {
                         T theta = (aqq - app) / (T(2) * apq);
                         T t;
-                        if (fabs(theta) > T(sizeof(T) == 8 ? 1e150 : 1e18))
+                        if (fabs(theta) > T(1e18))
                             t = T(0.5) / theta;
                         else
                             t = (theta >= T(0) ? T(1) : T(-1)) / (fabs(theta) + sqrt(T(1) + theta * theta));
@@ -130,6 +131,156 @@ __device__ void jacobi_eigen(T *A, T *V, int R, T *csbuf, int *pqbuf, int *flag)
             __syncthreads();
         }
         if (*flag == 0) break;
+        __syncthreads();
+    }
+    __syncthreads();
+}
+
+// ------------------------------------------------------------ FP64 Jacobi
+
+// Jacobi rotation of the pair (p, q) in FP64: c, s with c^2 + s^2 = 1 to FP64
+// accuracy and t = s / c the small-angle solution of t^2 + 2 theta t - 1 = 0,
+// theta = (a_qq - a_pp) / (2 a_pq), to FP32 accuracy: the rotation leaves
+// about 2^-23 |a_pq| of the entry, which the next sweep removes with the
+// second-order rest.  Returns false (no rotation) when |a_pq| <= 2^-53
+// sqrt(|a_pp a_qq|).  A division or square root on GB300's FP64 pipe is some
+// ten instructions of 64 cycles each; t comes from FP32 values scaled by a
+// common power of two, c from an FP32 reciprocal square root and two Newton
+// steps c <- c (3 - (1 + t^2) c^2) / 2 in FP64.
+__device__ __forceinline__ bool rotation64(double app, double aqq, double apq, double &c, double &s) {
+    c = 1.0;
+    s = 0.0;
+    const int ep = (__double2hiint(app) >> 20) & 0x7ff, eq = (__double2hiint(aqq) >> 20) & 0x7ff,
+              eo = (__double2hiint(apq) >> 20) & 0x7ff;
+    const int em = max(max(ep, eq), eo);
+    if (eo == 0 || em >= 2047) return false;  // zero or subnormal entry, infinities, NaN
+    const int sh = max(1, min(2045, 2046 - em));
+    const double sc = __hiloint2double(sh << 20, 0);  // 2^(1023 - em): the largest in [1, 2)
+    const double p = app * sc, q = aqq * sc, o = apq * sc;
+    if (!(o * o > 1.2325951644078309e-32 * fabs(p * q))) return false;  // 2^-106
+    const float d = d2f_rn(q - p), b = 2.0f * d2f_rn(o);
+    if (b == 0.0f) return false;
+    const float tf = fabsf(b) / (fabsf(d) + sqrtf(fmaf(d, d, b * b)));  // theta = d / b
+    const double t = (double)((d < 0.0f) == (b < 0.0f) ? tf : -tf);
+    const double w = fma(t, t, 1.0);
+    double x = (double)rsqrtf((float)w);
+    x = x * fma(-0.5 * w * x, x, 1.5);
+    x = x * fma(-0.5 * w * x, x, 1.5);
+    c = x;
+    s = t * x;
+    return true;
+}
+
+// Storage of a matrix the Jacobi method works on: shared (or this CTA's own
+// global) memory, or global memory shared by the CTAs of a cluster, which is
+// read and written in L2.
+struct OwnMat {
+    double *p;
+    __device__ __forceinline__ double ld(int e) const { return p[e]; }
+    __device__ __forceinline__ void st(int e, double v) const { p[e] = v; }
+};
+struct ClusterMat {
+    double *p;
+    __device__ __forceinline__ double ld(int e) const { return __ldcg(p + e); }
+    __device__ __forceinline__ void st(int e, double v) const { __stcg(p + e, v); }
+};
+
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+template <bool CL>
+__device__ __forceinline__ void team_sync() {
+    if constexpr (CL) cluster_sync();
+    else __syncthreads();
+}
+
+// The two-sided Jacobi method in FP64 by one CTA, or by the nr CTAs of a cluster (CL; this
+// one is number rk): eigenvalues on the diagonal of A, eigenvectors in V's
+// columns.  Only A's upper triangle is read and written.  A round's work --
+// the 2 x 2 blocks (pair i, pair k >= i) of A and the column pairs of V -- is
+// split over all threads; every CTA forms all the round's rotations itself
+// from the same entries, so the CTAs agree on them without an exchange.
+// Scratch per CTA: cs (R + 2 doubles), pq (R + 2 ints), flag.
+template <bool CL, class MA, class MV>
+__device__ inline void jacobi64(const MA A, const MV V, int R, double *cs, int *pq, int *flag, int rk, int nr) {
+    const int tid = threadIdx.x, nth = blockDim.x;
+    const int n = R + (R & 1), half = n / 2;
+    const int first = rk * nth + tid, stride = nr * nth;
+    auto at = [&](int r, int c) { return r < c ? r * R + c : c * R + r; };
+    for (int e = first; e < R * R; e += stride) V.st(e, (e / R == e % R) ? 1.0 : 0.0);
+    if (tid == 0) *flag = 0;
+    team_sync<CL>();
+    const int ntri = half * (half + 1) / 2;
+    const int nvp = half * R;
+    for (int sweep = 0; sweep < 40; ++sweep) {
+        for (int round = 0; round < n - 1; ++round) {
+            for (int i = tid; i < half; i += nth) {
+                int p, q;
+                if (i == 0) {
+                    p = round;
+                    q = n - 1;
+                } else {
+                    p = (round + i) % (n - 1);
+                    q = (round - i + (n - 1)) % (n - 1);
+                }
+                if (p > q) {
+                    const int t = p;
+                    p = q;
+                    q = t;
+                }
+                double c = 1.0, s = 0.0;
+                if (q < R && rotation64(A.ld(p * R + p), A.ld(q * R + q), A.ld(p * R + q), c, s)) *flag = 1;
+                cs[2 * i] = c;
+                cs[2 * i + 1] = s;
+                pq[2 * i] = p;
+                pq[2 * i + 1] = q;
+            }
+            team_sync<CL>();  // no CTA changes A while another still reads the round's entries
+            for (int w = first; w < ntri + nvp; w += stride) {
+                if (w < ntri) {
+                    // block (i, k), k >= i: row i of the triangle starts at i half - i (i - 1) / 2
+                    const float f = (float)(2 * half + 1);
+                    int i = min(half - 1, max(0, (int)((f - sqrtf(f * f - 8.0f * (float)w)) * 0.5f)));
+                    while (i + 1 < half && packed_row_offset(i + 1, half) <= w) ++i;
+                    while (packed_row_offset(i, half) > w) --i;
+                    const int k = i + w - packed_row_offset(i, half);
+                    const double si = cs[2 * i + 1], sk = cs[2 * k + 1];
+                    if (si == 0.0 && sk == 0.0) continue;
+                    const double ci = cs[2 * i], ck = cs[2 * k];
+                    const int pi = pq[2 * i], qi = pq[2 * i + 1], pk = pq[2 * k], qk = pq[2 * k + 1];
+                    const bool rq = qi < R, cq = qk < R;  // the padding index of odd R has no storage
+                    double x00 = A.ld(at(pi, pk));
+                    double x01 = cq ? A.ld(at(pi, qk)) : 0.0;
+                    double x10 = i == k ? x01 : (rq ? A.ld(at(qi, pk)) : 0.0);
+                    double x11 = (rq && cq) ? A.ld(at(qi, qk)) : 0.0;
+                    const double t00 = ck * x00 - sk * x01, t01 = sk * x00 + ck * x01;
+                    const double t10 = ck * x10 - sk * x11, t11 = sk * x10 + ck * x11;
+                    x00 = ci * t00 - si * t10;
+                    x10 = si * t00 + ci * t10;
+                    x01 = ci * t01 - si * t11;
+                    x11 = si * t01 + ci * t11;
+                    A.st(at(pi, pk), x00);
+                    if (cq) A.st(at(pi, qk), x01);
+                    if (rq && i != k) A.st(at(qi, pk), x10);
+                    if (rq && cq) A.st(at(qi, qk), x11);
+                } else {
+                    const int w2 = w - ntri, k = w2 / R, r = w2 - k * R;
+                    const double sk = cs[2 * k + 1];
+                    if (sk == 0.0) continue;
+                    const double ck = cs[2 * k];
+                    const int pk = pq[2 * k], qk = pq[2 * k + 1];
+                    const double vp = V.ld(r * R + pk), vq = V.ld(r * R + qk);
+                    V.st(r * R + pk, ck * vp - sk * vq);
+                    V.st(r * R + qk, sk * vp + ck * vq);
+                }
+            }
+            team_sync<CL>();
+        }
+        const int any = *flag;
+        __syncthreads();
+        if (tid == 0) *flag = 0;
+        if (!any) break;
         __syncthreads();
     }
     __syncthreads();
