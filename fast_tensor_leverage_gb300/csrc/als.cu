@@ -382,7 +382,7 @@ __global__ void pinv_square_kernel(const double *__restrict__ M, int R, int targ
         A[e] = a <= b ? M[e] : M[b * R + a];
     }
     __syncthreads();
-    jacobi64<false>(OwnMat{A}, OwnMat{V}, R, cs, pq, flag, 0, 1);
+    jacobi64(A, V, R, cs, pq, flag);
     sort_ascending<double>(A, R, order);
     for (int e = tid; e < RR; e += nth) {
         int a = e / R, b = e - a * R;
@@ -778,14 +778,6 @@ __device__ __forceinline__ void fiber_normals(uint64_t seed, uint32_t mode, uint
     sincospif(2.0f * u2, &sn, &cs);
     z0 = r * cs;
     z1 = r * sn;
-}
-
-// (double)x for a finite x that is zero or normal, by integer operations: the
-// conversion runs on the FP64 pipe, where a warp instruction takes 64 cycles.
-__device__ __forceinline__ double f2d_exact(float x) {
-    const uint32_t b = __float_as_uint(x), a = b & 0x7fffffffu;
-    const uint32_t hi = (b & 0x80000000u) | (a ? (a >> 3) + 0x38000000u : 0u);
-    return __hiloint2double((int)hi, (int)(b << 29));
 }
 
 // out[idx_j(z), :] += val(z) * g(fiber(z)) over the nonzeros sorted by their

@@ -170,7 +170,7 @@ __global__ void computem_pinv_kernel(CMParams p) {
     if (!chol) {
     for (int e = tid; e < RR; e += nth) A[e] = p.M[e];
     __syncthreads();
-    jacobi64<false>(OwnMat{A}, OwnMat{V}, R, cs, pq, flag, 0, 1);
+    jacobi64(A, V, R, cs, pq, flag);
     sort_ascending<double>(A, R, order);
     // W = M[N]: row (R-1-r) = v_r / sqrt(lambda_r) for lambda_r > 1e-8, else 0,
     // r the ascending rank (column R-1-r of the reference's V Lambda^{-1/2}).
@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(FTL_CM_THREADS) computem_eig_kernel(CMParams p
     } else if (offset < N) {
         for (int e = tid; e < RR; e += nth) A[e] = W[e];
         __syncthreads();
-        jacobi64<false>(OwnMat{A}, OwnMat{V}, R, cs, pq, flag, 0, 1);
+        jacobi64(A, V, R, cs, pq, flag);
         sort_ascending<double>(A, R, order);
         // row r = sqrt(lambda_r) v_r, ascending (negative rounding noise -> 0)
         for (int e = tid; e < RR; e += nth) {
@@ -415,14 +415,15 @@ __global__ void __launch_bounds__(FTL_CM_THREADS) computem_eig_kernel(CMParams p
 //
 // One CTA has an SM's FP64 pipe: two lanes per cycle.  A Jacobi round at R =
 // 100 is 40,000 FP64 lane operations and the two eigensolves took 19.2 and
-// 19.8 ms.  A cluster of eight CTAs shares one matrix in L2 (A in its M slot,
-// V in its scratch slot); every other step is split over the cluster's threads
+// 19.8 ms.  A cluster of eight CTAs shares one matrix in L2 (A in its M slot);
+// every other step is split over the cluster's threads
 // so that an entry stays with one thread and needs no exchange.
 constexpr int kCmCluster = 8;
 constexpr int kCmClThreads = 512;
 
 struct CMClShared {
     double cs[FTL_MAX_RANK + 2], lam[FTL_MAX_RANK];
+    double V[FTL_MAX_RANK / kCmCluster * FTL_MAX_RANK];  // this CTA's rows of the eigenvectors
     int pq[FTL_MAX_RANK + 2], order[FTL_MAX_RANK], flag;
 };
 
@@ -463,9 +464,10 @@ __global__ void __cluster_dims__(kCmCluster, 1, 1) __launch_bounds__(kCmClThread
     }
     if (first == 0) p.M[cm_status_offset(N, R)] = 0.0;
     cluster_sync();
-    const ClusterMat A{p.M}, V{p.M + (size_t)(N + 2) * RR};
-    jacobi64<true>(A, V, R, sm.cs, sm.pq, &sm.flag, rk, kCmCluster);
-    cl_sort(sm, A, R);
+    double *eig, *vec;
+    jacobi64_cluster(p.M, p.M + (size_t)(N + 2) * RR, R, sm.cs, sm.pq, &sm.flag, sm.V, rk, kCmCluster, &eig, &vec);
+    const ClusterMat V{vec};
+    cl_sort(sm, ClusterMat{eig}, R);
     // W = M[N]: row (R-1-r) = v_r / sqrt(lambda_r) for lambda_r > 1e-8, else 0
     double *W = p.M + (size_t)N * RR;
     for (int e = first; e < RR; e += stride) {
@@ -509,15 +511,21 @@ __global__ void __cluster_dims__(kCmCluster, 1, 1) __launch_bounds__(kCmClThread
     const int offset = ((uint32_t)(k + 1) == p.j) ? k + 2 : k + 1;
     double *W = p.M + (size_t)offset * RR;
     if (offset < N) {
-        const ClusterMat A{W}, V{p.M + (size_t)(N + 3 + k) * RR};
-        jacobi64<true>(A, V, R, sm.cs, sm.pq, &sm.flag, rk, kCmCluster);
-        cl_sort(sm, A, R);
-        cluster_sync();  // every CTA has the eigenvalues: A's slot can be overwritten
+        double *eig, *vec, *other = p.M + (size_t)(N + 3 + k) * RR;
+        jacobi64_cluster(W, other, R, sm.cs, sm.pq, &sm.flag, sm.V, rk, kCmCluster, &eig, &vec);
+        const ClusterMat V{vec};
+        cl_sort(sm, ClusterMat{eig}, R);
+        cluster_sync();  // every CTA has the eigenvalues: their copy can be overwritten
         // row r = sqrt(lambda_r) v_r, ascending (negative rounding noise -> 0)
+        double *rows = vec == W ? other : W;
         for (int e = first; e < RR; e += stride) {
             const int r = e / R, a = e - r * R;
             const int v = sm.order[r];
-            __stcg(W + e, sqrt(fmax(sm.lam[v], 0.0)) * V.ld(a * R + v));
+            __stcg(rows + e, sqrt(fmax(sm.lam[v], 0.0)) * V.ld(a * R + v));
+        }
+        if (rows != W) {  // the draws read the rows from W's slot
+            cluster_sync();
+            for (int e = first; e < RR; e += stride) __stcg(W + e, __ldcg(rows + e));
         }
         if (rk == 0)
             for (int r = threadIdx.x; r < R; r += blockDim.x) p.lambda[(size_t)offset * R + r] = sm.lam[sm.order[r]];

@@ -145,8 +145,9 @@ __device__ inline void jacobi_eigen32(float *A, float *V, int R, float *csbuf, i
 // second-order rest.  Returns false (no rotation) when |a_pq| <= 2^-53
 // sqrt(|a_pp a_qq|).  A division or square root on GB300's FP64 pipe is some
 // ten instructions of 64 cycles each; t comes from FP32 values scaled by a
-// common power of two, c from an FP32 reciprocal square root and two Newton
-// steps c <- c (3 - (1 + t^2) c^2) / 2 in FP64.
+// common power of two, c from an FP32 reciprocal square root x of 1 + t^2 and
+// one third-order step, c = x + x e (1/2 + 3/8 e) with e = 1 - (1 + t^2) x^2
+// (the series of (1 - e)^(-1/2): 2^-22 becomes below 2^-60).
 __device__ __forceinline__ bool rotation64(double app, double aqq, double apq, double &c, double &s) {
     c = 1.0;
     s = 0.0;
@@ -161,13 +162,11 @@ __device__ __forceinline__ bool rotation64(double app, double aqq, double apq, d
     const float d = d2f_rn(q - p), b = 2.0f * d2f_rn(o);
     if (b == 0.0f) return false;
     const float tf = fabsf(b) / (fabsf(d) + sqrtf(fmaf(d, d, b * b)));  // theta = d / b
-    const double t = (double)((d < 0.0f) == (b < 0.0f) ? tf : -tf);
-    const double w = fma(t, t, 1.0);
-    double x = (double)rsqrtf((float)w);
-    x = x * fma(-0.5 * w * x, x, 1.5);
-    x = x * fma(-0.5 * w * x, x, 1.5);
-    c = x;
-    s = t * x;
+    const double t = f2d_exact((d < 0.0f) == (b < 0.0f) ? tf : -tf);
+    const double w = fma(t, t, 1.0), x = f2d_exact(rsqrtf(fmaf(tf, tf, 1.0f)));
+    const double e = fma(-w * x, x, 1.0);
+    c = fma(x * e, fma(0.375, e, 0.5), x);
+    s = t * c;
     return true;
 }
 
@@ -189,93 +188,98 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-template <bool CL>
-__device__ __forceinline__ void team_sync() {
-    if constexpr (CL) cluster_sync();
-    else __syncthreads();
+// Pair i of a round-robin round over n (even) indices, p < q.
+__device__ __forceinline__ void jacobi_pair(int round, int i, int n, int &p, int &q) {
+    p = i == 0 ? round : (round + i) % (n - 1);
+    q = i == 0 ? n - 1 : (round - i + (n - 1)) % (n - 1);
+    if (p > q) {
+        const int t = p;
+        p = q;
+        q = t;
+    }
 }
 
-// The two-sided Jacobi method in FP64 by one CTA, or by the nr CTAs of a cluster (CL; this
-// one is number rk): eigenvalues on the diagonal of A, eigenvectors in V's
-// columns.  Only A's upper triangle is read and written.  A round's work --
-// the 2 x 2 blocks (pair i, pair k >= i) of A and the column pairs of V -- is
-// split over all threads; every CTA forms all the round's rotations itself
-// from the same entries, so the CTAs agree on them without an exchange.
-// Scratch per CTA: cs (R + 2 doubles), pq (R + 2 ints), flag.
-template <bool CL, class MA, class MV>
-__device__ inline void jacobi64(const MA A, const MV V, int R, double *cs, int *pq, int *flag, int rk, int nr) {
+// Block (i, k), k >= i, number w of the triangle of `half` pairs: row i starts
+// at i half - i (i - 1) / 2.
+__device__ __forceinline__ void jacobi_block(int w, int half, int &i, int &k) {
+    const float f = (float)(2 * half + 1);
+    i = min(half - 1, max(0, (int)((f - sqrtf(f * f - 8.0f * (float)w)) * 0.5f)));
+    while (i + 1 < half && packed_row_offset(i + 1, half) <= w) ++i;
+    while (packed_row_offset(i, half) > w) --i;
+    k = i + w - packed_row_offset(i, half);
+}
+
+// The round's rotations of all pairs, from the matrix A.
+template <class MA>
+__device__ __forceinline__ void jacobi_rotations(const MA A, int R, int round, double *cs, int *pq, int *flag) {
+    const int n = R + (R & 1);
+    for (int i = threadIdx.x; i < n / 2; i += blockDim.x) {
+        int p, q;
+        jacobi_pair(round, i, n, p, q);
+        double c = 1.0, s = 0.0;
+        if (q < R && rotation64(A.ld(p * R + p), A.ld(q * R + q), A.ld(p * R + q), c, s)) *flag = 1;
+        cs[2 * i] = c;
+        cs[2 * i + 1] = s;
+        pq[2 * i] = p;
+        pq[2 * i + 1] = q;
+    }
+}
+
+// One 2 x 2 block of the round from A into B (A and B may be the same).
+template <class MA>
+__device__ __forceinline__ void jacobi_rotate(const MA A, const MA B, int R, int i, int k, const double *cs,
+                                              const int *pq) {
+    auto at = [&](int r, int c) { return r < c ? r * R + c : c * R + r; };
+    const double ci = cs[2 * i], si = cs[2 * i + 1], ck = cs[2 * k], sk = cs[2 * k + 1];
+    const int pi = pq[2 * i], qi = pq[2 * i + 1], pk = pq[2 * k], qk = pq[2 * k + 1];
+    const bool rq = qi < R, cq = qk < R;  // the padding index of odd R has no storage
+    double x00 = A.ld(at(pi, pk));
+    double x01 = cq ? A.ld(at(pi, qk)) : 0.0;
+    double x10 = i == k ? x01 : (rq ? A.ld(at(qi, pk)) : 0.0);
+    double x11 = (rq && cq) ? A.ld(at(qi, qk)) : 0.0;
+    const double t00 = ck * x00 - sk * x01, t01 = sk * x00 + ck * x01;
+    const double t10 = ck * x10 - sk * x11, t11 = sk * x10 + ck * x11;
+    x00 = ci * t00 - si * t10;
+    x10 = si * t00 + ci * t10;
+    x01 = ci * t01 - si * t11;
+    x11 = si * t01 + ci * t11;
+    B.st(at(pi, pk), x00);
+    if (cq) B.st(at(pi, qk), x01);
+    if (rq && i != k) B.st(at(qi, pk), x10);
+    if (rq && cq) B.st(at(qi, qk), x11);
+}
+
+// The two-sided Jacobi method in FP64 by one CTA: eigenvalues on the diagonal
+// of A, eigenvectors in V's columns.  Only A's upper triangle is read and
+// written.  Scratch: cs (R + 2 doubles), pq (R + 2 ints), flag.
+__device__ inline void jacobi64(double *A, double *V, int R, double *cs, int *pq, int *flag) {
     const int tid = threadIdx.x, nth = blockDim.x;
     const int n = R + (R & 1), half = n / 2;
-    const int first = rk * nth + tid, stride = nr * nth;
-    auto at = [&](int r, int c) { return r < c ? r * R + c : c * R + r; };
-    for (int e = first; e < R * R; e += stride) V.st(e, (e / R == e % R) ? 1.0 : 0.0);
+    const OwnMat M{A};
+    for (int e = tid; e < R * R; e += nth) V[e] = (e / R == e % R) ? 1.0 : 0.0;
     if (tid == 0) *flag = 0;
-    team_sync<CL>();
-    const int ntri = half * (half + 1) / 2;
-    const int nvp = half * R;
+    __syncthreads();
+    const int ntri = half * (half + 1) / 2, nvp = half * R;
     for (int sweep = 0; sweep < 40; ++sweep) {
         for (int round = 0; round < n - 1; ++round) {
-            for (int i = tid; i < half; i += nth) {
-                int p, q;
-                if (i == 0) {
-                    p = round;
-                    q = n - 1;
-                } else {
-                    p = (round + i) % (n - 1);
-                    q = (round - i + (n - 1)) % (n - 1);
-                }
-                if (p > q) {
-                    const int t = p;
-                    p = q;
-                    q = t;
-                }
-                double c = 1.0, s = 0.0;
-                if (q < R && rotation64(A.ld(p * R + p), A.ld(q * R + q), A.ld(p * R + q), c, s)) *flag = 1;
-                cs[2 * i] = c;
-                cs[2 * i + 1] = s;
-                pq[2 * i] = p;
-                pq[2 * i + 1] = q;
-            }
-            team_sync<CL>();  // no CTA changes A while another still reads the round's entries
-            for (int w = first; w < ntri + nvp; w += stride) {
+            jacobi_rotations(M, R, round, cs, pq, flag);
+            __syncthreads();
+            for (int w = tid; w < ntri + nvp; w += nth) {
                 if (w < ntri) {
-                    // block (i, k), k >= i: row i of the triangle starts at i half - i (i - 1) / 2
-                    const float f = (float)(2 * half + 1);
-                    int i = min(half - 1, max(0, (int)((f - sqrtf(f * f - 8.0f * (float)w)) * 0.5f)));
-                    while (i + 1 < half && packed_row_offset(i + 1, half) <= w) ++i;
-                    while (packed_row_offset(i, half) > w) --i;
-                    const int k = i + w - packed_row_offset(i, half);
-                    const double si = cs[2 * i + 1], sk = cs[2 * k + 1];
-                    if (si == 0.0 && sk == 0.0) continue;
-                    const double ci = cs[2 * i], ck = cs[2 * k];
-                    const int pi = pq[2 * i], qi = pq[2 * i + 1], pk = pq[2 * k], qk = pq[2 * k + 1];
-                    const bool rq = qi < R, cq = qk < R;  // the padding index of odd R has no storage
-                    double x00 = A.ld(at(pi, pk));
-                    double x01 = cq ? A.ld(at(pi, qk)) : 0.0;
-                    double x10 = i == k ? x01 : (rq ? A.ld(at(qi, pk)) : 0.0);
-                    double x11 = (rq && cq) ? A.ld(at(qi, qk)) : 0.0;
-                    const double t00 = ck * x00 - sk * x01, t01 = sk * x00 + ck * x01;
-                    const double t10 = ck * x10 - sk * x11, t11 = sk * x10 + ck * x11;
-                    x00 = ci * t00 - si * t10;
-                    x10 = si * t00 + ci * t10;
-                    x01 = ci * t01 - si * t11;
-                    x11 = si * t01 + ci * t11;
-                    A.st(at(pi, pk), x00);
-                    if (cq) A.st(at(pi, qk), x01);
-                    if (rq && i != k) A.st(at(qi, pk), x10);
-                    if (rq && cq) A.st(at(qi, qk), x11);
+                    int i, k;
+                    jacobi_block(w, half, i, k);
+                    if (cs[2 * i + 1] != 0.0 || cs[2 * k + 1] != 0.0) jacobi_rotate(M, M, R, i, k, cs, pq);
                 } else {
                     const int w2 = w - ntri, k = w2 / R, r = w2 - k * R;
-                    const double sk = cs[2 * k + 1];
+                    const double ck = cs[2 * k], sk = cs[2 * k + 1];
                     if (sk == 0.0) continue;
-                    const double ck = cs[2 * k];
-                    const int pk = pq[2 * k], qk = pq[2 * k + 1];
-                    const double vp = V.ld(r * R + pk), vq = V.ld(r * R + qk);
-                    V.st(r * R + pk, ck * vp - sk * vq);
-                    V.st(r * R + qk, sk * vp + ck * vq);
+                    const int pk = r * R + pq[2 * k], qk = r * R + pq[2 * k + 1];
+                    const double vp = V[pk], vq = V[qk];
+                    V[pk] = ck * vp - sk * vq;
+                    V[qk] = sk * vp + ck * vq;
                 }
             }
-            team_sync<CL>();
+            __syncthreads();
         }
         const int any = *flag;
         __syncthreads();
@@ -284,6 +288,61 @@ __device__ inline void jacobi64(const MA A, const MV V, int R, double *cs, int *
         __syncthreads();
     }
     __syncthreads();
+}
+
+// The same by the nr CTAs of a cluster (this one is number rk), on two copies
+// of the matrix in global memory: a round reads one and writes every block into
+// the other, so that one barrier per round is enough.  The blocks are split
+// over all threads; every CTA forms all the round's rotations itself from the
+// same entries, so the CTAs agree on them without an exchange; a CTA keeps its
+// ceil(R / nr) rows of V in shared memory (Vs) and rotates them between
+// arriving at the barrier and waiting.  A0 holds the matrix; on return *eig
+// points to the copy with the eigenvalues on its diagonal and *vec to the
+// other one, which holds V.
+__device__ inline void jacobi64_cluster(double *A0, double *A1, int R, double *cs, int *pq, int *flag, double *Vs,
+                                        int rk, int nr, double **eig, double **vec) {
+    const int tid = threadIdx.x, nth = blockDim.x;
+    const int n = R + (R & 1), half = n / 2;
+    const int rpc = (R + nr - 1) / nr, r0 = rk * rpc, nrows = max(0, min(R, r0 + rpc) - r0);
+    for (int e = tid; e < nrows * R; e += nth) Vs[e] = (r0 + e / R == e % R) ? 1.0 : 0.0;
+    if (tid == 0) *flag = 0;
+    cluster_sync();
+    const int ntri = half * (half + 1) / 2;
+    ClusterMat src{A0}, dst{A1};
+    for (int sweep = 0; sweep < 40; ++sweep) {
+        for (int round = 0; round < n - 1; ++round) {
+            jacobi_rotations(src, R, round, cs, pq, flag);
+            __syncthreads();
+            for (int w = rk + nr * tid; w < ntri; w += nr * nth) {  // every CTA the same share
+                int i, k;
+                jacobi_block(w, half, i, k);
+                jacobi_rotate(src, dst, R, i, k, cs, pq);
+            }
+            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+            for (int w = tid; w < half * nrows; w += nth) {
+                const int k = w / nrows, r = w - k * nrows;
+                const double ck = cs[2 * k], sk = cs[2 * k + 1];
+                if (sk == 0.0) continue;
+                const int pk = r * R + pq[2 * k], qk = r * R + pq[2 * k + 1];
+                const double vp = Vs[pk], vq = Vs[qk];
+                Vs[pk] = ck * vp - sk * vq;
+                Vs[qk] = sk * vp + ck * vq;
+            }
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+            const ClusterMat t = src;
+            src = dst;
+            dst = t;
+        }
+        const int any = *flag;
+        __syncthreads();
+        if (tid == 0) *flag = 0;
+        if (!any) break;
+        __syncthreads();
+    }
+    for (int e = tid; e < nrows * R; e += nth) dst.st(r0 * R + e, Vs[e]);
+    cluster_sync();
+    *eig = src.p;
+    *vec = dst.p;
 }
 
 // order[r] = index of the r-th smallest eigenvalue (ties by index).

@@ -193,6 +193,14 @@ __device__ __forceinline__ float d2f_rn(double x) {
     return __double2float_rn(x);
 }
 
+// (double)x for a finite x that is zero or normal, by integer operations: the
+// conversion runs on the FP64 pipe, where a warp instruction takes 64 cycles.
+__device__ __forceinline__ double f2d_exact(float x) {
+    const uint32_t b = __float_as_uint(x), a = b & 0x7fffffffu;
+    const uint32_t hi = (b & 0x80000000u) | (a ? (a >> 3) + 0x38000000u : 0u);
+    return __hiloint2double((int)hi, (int)(b << 29));
+}
+
 // ------------------------------------------------------------------ warps
 
 template <typename T>
