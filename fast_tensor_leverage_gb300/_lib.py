@@ -102,6 +102,8 @@ SIGNATURES = {
     "ftl_lowrank_mttkrp_workspace_bytes": ([_INT, _INT, _P], _INT),
     "ftl_lowrank_sampled_mttkrp": ([_P, _P, _INT, _INT, _INT, _P, _I64, _P, _P, _P, _I64, _P, _P, _INT, _P,
                                     ctypes.c_size_t, _P, _I64, _I64, _P], _INT),
+    "ftl_lowrank_sampled_solve": ([_P, _P, _INT, _INT, _INT, _P, _I64, _P, _P, _P, _I64, _P, _P, _INT, _P, _P,
+                                  ctypes.c_size_t, _P, _I64, _I64, _P], _INT),
     "ftl_dense_sampled_mttkrp": ([_P, _INT, _P, _INT, _INT, _P, _I64, _P, _P, _P, _I64, _P, _P, _INT, _P, _I64,
                                   _P], _INT),
     "ftl_dense_materialize": ([_P, _INT, _P, _INT, _INT, _P, _I64, _P, _P], _INT),
@@ -156,6 +158,7 @@ SIGNATURES = {
     "ftl_sparse_residual_terms": ([_P, _P, _I64, _INT, _P, _P, _INT, _P, ctypes.c_size_t, _P, _P], _INT),
     "ftl_sum_squares": ([_P, _I64, _P, ctypes.c_size_t, _P, _P], _INT),
     "ftl_sparse_exact_mttkrp": ([_P, _P, _I64, _INT, _INT, _P, _INT, _P, _I64, _P], _INT),
+    "ftl_solve_rows_at": ([_P, _P, _P, _P, _I64, _INT, _P, _P], _INT),
     "ftl_sparse_exact_mttkrp_rows": ([_P, _P, _P, _I64, _INT, _P, _INT, _P, _INT, _P, _I64, _P], _INT),
     "ftl_gram_hadamard": ([_P, _INT, _INT, _INT, _P, _P, _P, _P, _P], _INT),
     "ftl_krp_sample_packed": ([_P, _INT, _P, _P, _P, _P, _P, _P, _P, _P], _INT),

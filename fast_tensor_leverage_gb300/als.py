@@ -115,13 +115,23 @@ class ALS:
                   self._pinv.data_ptr(), self._vscr.data_ptr(), st)
         I_j = lr.dims[j]
         # U_j = MTTKRP pinv (als.hpp:189-203) with MTTKRP = sum_z coef_z e_row(z)
-        # h_rep(z)^T, i.e. U_j = sum_z coef_z e_row(z) (h_rep(z)^T pinv): the J
-        # sampled rows are multiplied by pinv first (J x R^2 FP64 instead of
-        # I_j x R^2) and the MTTKRP accumulates straight into U_j.
+        # h_rep(z)^T, i.e. U_j = sum_z coef_z e_row(z) (h_rep(z)^T pinv): the
+        # unique sampled rows are multiplied by pinv first (at most J x R^2
+        # FP64 instead of I_j x R^2) and the MTTKRP accumulates straight into
+        # U_j; against a low-rank tensor the product in its middle is.
         hp = self._hp
-        _lib.call("ftl_solve_rows", h.data_ptr(), self._pinv.data_ptr(), J, R, hp.data_ptr(), st)
         out = lr.U_dev[j]
-        if not isinstance(gt, SparseTensor):
+        in_middle = isinstance(gt, LowRankTensor) and not gt.noise_sigma
+        if in_middle:
+            gt._sampled_solve_dev(samples.data_ptr(), J, self._urep.data_ptr(), self._ucnt.data_ptr(),
+                                  self._nuniq.data_ptr(), w.data_ptr(), h.data_ptr(), self._pinv.data_ptr(), R, j,
+                                  out.data_ptr(), I_j, st)
+        else:
+            _lib.call("ftl_solve_rows_at", h.data_ptr(), self._pinv.data_ptr(), self._urep.data_ptr(),
+                      self._nuniq.data_ptr(), J, R, hp.data_ptr(), st)
+        if in_middle:
+            pass
+        elif not isinstance(gt, SparseTensor):
             # black-box right-hand side (black_box_tensor.hpp:21-67): low-rank
             # shortcut or dense fiber gather, rows past gt.dims[j] zeroed
             gt._sampled_mttkrp_dev(samples.data_ptr(), J, self._urep.data_ptr(), self._ucnt.data_ptr(),

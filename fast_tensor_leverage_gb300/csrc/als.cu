@@ -205,15 +205,25 @@ static int64_t table_size_for(int64_t J) {
 // partial[b][e] = sum over this block's rows u of s_u * h_a h_b, e = packed
 // (a, b); rows u < *n_rows (or n_rows_host), h row = lhs[row(u)], s_u =
 // (w ? w[row(u)] : 1) * (cnt ? cnt[u] : 1).  Rows are staged 32 at a time
-// with their scaled copy s_u h; each thread owns up to GRAM_EPT packed
-// entries (thread t: entries t, t + blockDim, ...; up to 9 covers R = 128,
-// 8256 entries, on 1024 threads) and adds one FMA per
-// entry and row.  All-zero rows are skipped (they add exact zeros): most
+// with their scaled copy s_u h (one copy when neither w nor cnt is given);
+// each thread owns up to GRAM_EPT packed entries (thread t: entries t,
+// t + blockDim, ...; up to 9 covers R = 128, 8256 entries) and adds one FMA
+// per entry and row.  All-zero rows are skipped (they add exact zeros): most
 // rows of a sampled-ALS factor are zero, and this is FP64 arithmetic at a
-// low issue rate.
-static int gram_threads(int R) {
-    const int P = packed_size(R);
-    return std::min(1024, (P + 31) / 32 * 32);
+// low issue rate.  The entries per thread are chosen so that a block has at
+// most 20 warps with few idle lanes (R = 64: 13 warps x 5 entries = 65 x 32),
+// and up to four blocks run per SM, so that one's staging overlaps another's
+// multiply-adds: 131,072 rows at R = 64 1.07 -> 0.53 ms, 1.4e6 rows at R = 25
+// 1.48 -> 0.86 ms against one block per SM.
+constexpr int kGramBlocks = 4;  // blocks per SM at most
+
+static void gram_shape(int R, int &ept, int &threads) {
+    const int w32 = (packed_size(R) + 31) / 32;
+    for (int e : {1, 2, 3, 5, 8, 9}) {
+        ept = e;
+        threads = (w32 + e - 1) / e * 32;
+        if (threads <= 20 * 32) break;
+    }
 }
 
 template <int GRAM_EPT>
@@ -227,7 +237,8 @@ __global__ void gram_partial_kernel(const double *__restrict__ lhs, const int32_
     const int64_t n = n_rows_dev ? *n_rows_dev : n_rows_host;
     const int64_t per = (n + gridDim.x - 1) / gridDim.x;
     const int64_t r0 = blockIdx.x * per, r1 = min(n, r0 + per);
-    double *hsc = hs + 32 * R;
+    const bool scaled = w || cnt;
+    double *hsc = scaled ? hs + 32 * R : hs;
     double acc[GRAM_EPT];
     int ea[GRAM_EPT], eb[GRAM_EPT];
 #pragma unroll
@@ -255,9 +266,8 @@ __global__ void gram_partial_kernel(const double *__restrict__ lhs, const int32_
             const int64_t u = u0 + uu;
             const int64_t row = rowidx ? rowidx[u] : u;
             const double v = lhs[row * R + (e - uu * R)];
-            const double su = (w ? w[row] : 1.0) * (cnt ? (double)cnt[u] : 1.0);
             hs[e] = v;
-            hsc[e] = su * v;
+            if (scaled) hsc[e] = (w ? w[row] : 1.0) * (cnt ? (double)cnt[u] : 1.0) * v;
             if (v != 0.0) nz[uu] = 1;
         }
         __syncthreads();
@@ -859,37 +869,103 @@ __global__ void __launch_bounds__(256) rrf_rows_kernel(const int32_t *__restrict
 
 // ------------------------------------------------------ solve / renorm
 
-// U = B pinv (pinv R x R symmetric) row by row; an all-zero row of B (a row
-// no sampled fiber touched) is written as zeros without arithmetic.
-__global__ void solve_rows_kernel(const double *__restrict__ B, const double *__restrict__ pinv, int64_t I, int R,
-                                  double *__restrict__ U) {
-    extern __shared__ double sm[];
-    double *ps = sm;               // R x R
-    double *bs = sm + R * R;       // blockDim.x rows x R (row-major)
-    for (int e = threadIdx.x; e < R * R; e += blockDim.x) ps[e] = pinv[e];
-    for (int64_t r0 = (int64_t)blockIdx.x * blockDim.x; r0 < I; r0 += (int64_t)gridDim.x * blockDim.x) {
-        const int m = (int)min((int64_t)blockDim.x, I - r0);
+// U = B pinv (pinv R x R symmetric) row by row, for all I rows or (rowidx) for
+// the rows rowidx[u], u < *n_dev; an all-zero row of B (a row no sampled fiber
+// touched) is written as zeros without arithmetic.  Bound by the FP64 pipe (R
+// multiply-adds per entry): a block stages TM rows and pinv in shared memory
+// and a thread owns 4 rows x TC columns, so that the pipe's four parts are all
+// fed from R = 100 on, where pinv alone takes 80 KB and one thread per row
+// left two of them idle.  The unique ones of 65,536 sampled rows at R = 100:
+// 3.40 (all rows, one thread per row) -> 1.04 ms.  TC = 5 where it divides R
+// and 4 does not.
+template <int TC>
+__global__ void solve_rows_kernel(const double *__restrict__ B, const double *__restrict__ pinv,
+                                  const int32_t *__restrict__ rowidx, const int64_t *__restrict__ n_dev, int64_t I,
+                                  int R, int TM, double *__restrict__ U) {
+    extern __shared__ __align__(16) double sm[];
+    const int ncg = (R + TC - 1) / TC, Rp = ncg * TC;
+    double *ps = sm;                           // R x Rp, zero padded
+    double *bs = sm + R * Rp;                  // TM rows x R
+    int *nz = (int *)(bs + TM * R);            // row has a nonzero entry
+    const int64_t n = n_dev ? min(I, *n_dev) : I;
+    for (int e = threadIdx.x; e < R * Rp; e += blockDim.x) {
+        const int k = e / Rp, c = e - k * Rp;
+        ps[e] = c < R ? pinv[k * R + c] : 0.0;
+    }
+    const int items = TM / 4 * ncg;
+    for (int64_t r0 = (int64_t)blockIdx.x * TM; r0 < n; r0 += (int64_t)gridDim.x * TM) {
+        const int m = (int)min((int64_t)TM, n - r0);
         __syncthreads();
-        for (int e = threadIdx.x; e < m * R; e += blockDim.x) bs[e] = B[r0 * R + e];
+        for (int r = threadIdx.x; r < TM; r += blockDim.x) nz[r] = 0;
         __syncthreads();
-        if (threadIdx.x < m) {
-            const double *b = bs + threadIdx.x * R;
-            bool any = false;
-            for (int c = 0; c < R; ++c) any |= (b[c] != 0.0);
-            double *o = bs + threadIdx.x * R;
-            if (any) {
-                double tmp[FTL_MAX_RANK];
-                for (int c = 0; c < R; ++c) tmp[c] = b[c];
-                for (int c = 0; c < R; ++c) {
-                    double s = 0.0;
-                    for (int k = 0; k < R; ++k) s = fma(tmp[k], ps[k * R + c], s);
-                    o[c] = s;
+        for (int e = threadIdx.x; e < TM * R; e += blockDim.x) {
+            const int r = e / R, c = e - r * R;
+            double v = 0.0;
+            if (r < m) {
+                const int64_t row = rowidx ? (int64_t)rowidx[r0 + r] : r0 + r;
+                v = B[row * R + c];
+            }
+            bs[e] = v;
+            if (v != 0.0) nz[r] = 1;
+        }
+        __syncthreads();
+        for (int w = threadIdx.x; w < items; w += blockDim.x) {
+            const int rg = 4 * (w / ncg), cg = TC * (w % ncg);
+            double acc[4][TC];
+#pragma unroll
+            for (int x = 0; x < 4; ++x)
+#pragma unroll
+                for (int y = 0; y < TC; ++y) acc[x][y] = 0.0;
+            if (nz[rg] | nz[rg + 1] | nz[rg + 2] | nz[rg + 3]) {
+                const double *b = bs + rg * R, *q = ps + cg;
+#pragma unroll 2
+                for (int k = 0; k < R; ++k) {
+                    double bv[4], pv[TC];
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) bv[x] = b[x * R + k];
+#pragma unroll
+                    for (int y = 0; y < TC; ++y) pv[y] = q[k * Rp + y];
+#pragma unroll
+                    for (int x = 0; x < 4; ++x)
+#pragma unroll
+                        for (int y = 0; y < TC; ++y) acc[x][y] = fma(bv[x], pv[y], acc[x][y]);
+                }
+            }
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                if (rg + x < m) {
+                    const int64_t row = rowidx ? (int64_t)rowidx[r0 + rg + x] : r0 + rg + x;
+#pragma unroll
+                    for (int y = 0; y < TC; ++y)
+                        if (cg + y < R) U[row * R + cg + y] = nz[rg + x] ? acc[x][y] : 0.0;
                 }
             }
         }
-        __syncthreads();
-        for (int e = threadIdx.x; e < m * R; e += blockDim.x) U[r0 * R + e] = bs[e];
     }
+}
+
+template <int TC>
+static int launch_solve_rows(const double *B, const double *pinv, const int32_t *rowidx, const int64_t *n_dev,
+                             int64_t I, int R, double *U, cudaStream_t st) {
+    const int ncg = (R + TC - 1) / TC;
+    const int TM = R <= 16 ? 256 : (R <= 32 ? 128 : 64);
+    const size_t smem = (size_t)(R * ncg * TC + TM * R) * sizeof(double) + TM * sizeof(int);
+    const int rc = ensure_smem((const void *)solve_rows_kernel<TC>, smem, "solve_rows_kernel");
+    if (rc) return rc;
+    const int threads = std::min(512, (TM / 4 * ncg + 31) / 32 * 32);
+    int occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, solve_rows_kernel<TC>, threads, smem) != cudaSuccess ||
+        occ < 1)
+        occ = 1;
+    const int blocks = (int)std::min<int64_t>((I + TM - 1) / TM, (int64_t)num_sms() * occ);
+    solve_rows_kernel<TC><<<blocks, threads, smem, st>>>(B, pinv, rowidx, n_dev, I, R, TM, U);
+    return check_launch("solve_rows_kernel");
+}
+
+static int solve_rows(const double *B, const double *pinv, const int32_t *rowidx, const int64_t *n_dev, int64_t I,
+                      int R, double *U, cudaStream_t st) {
+    if (R % 5 == 0 && R % 4 != 0) return launch_solve_rows<5>(B, pinv, rowidx, n_dev, I, R, U, st);
+    return launch_solve_rows<4>(B, pinv, rowidx, n_dev, I, R, U, st);
 }
 
 // Thread t owns column t % R of rows t / R, t / R + rows_per_pass, ... (a
@@ -920,9 +996,10 @@ __global__ void colsq_partial_kernel(const double *__restrict__ U, int64_t I, in
 // norms: sqrt of the column sums, <= 1e-7 -> 1 (low_rank_tensor.hpp:229-238);
 // one warp per column, lanes over the block partials.
 __global__ void colnorm_finish_kernel(const double *__restrict__ partial, int nblk, int R, double *__restrict__ norms) {
-    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int c = threadIdx.x >> 5; c < R; c += nw) {
+    const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
+    for (int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < R; c += nw) {
         double s = 0.0;
+#pragma unroll 8
         for (int k = lane; k < nblk; k += 32) s += partial[(int64_t)k * R + c];
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (lane == 0) {
@@ -1217,10 +1294,12 @@ __global__ void gram_hadamard_kernel(GramPtrs gp, int N, int R, int exclude, con
     }
     red[threadIdx.x] = acc;
     __syncthreads();
-    if (threadIdx.x == 0 && out_sum) {
+    // by one warp in a fixed order: 32 + 5 dependent FP64 additions, not 1024
+    if (threadIdx.x < 32 && out_sum) {
         double s = 0.0;
-        for (int t = 0; t < (int)blockDim.x; ++t) s += red[t];
-        *out_sum = s;
+        for (int t = threadIdx.x; t < (int)blockDim.x; t += 32) s += red[t];
+        s = warp_sum(s);
+        if (threadIdx.x == 0) *out_sum = s;
     }
 }
 
@@ -1360,7 +1439,7 @@ extern "C" int ftl_sparse_mttkrp_rows(const int32_t *row_idx, const uint64_t *ro
 
 extern "C" int ftl_gram_workspace_bytes(int R, size_t *out) {
     FTL_CHECK_ARG(out && R >= 1 && R <= FTL_MAX_RANK, "ftl_gram_workspace_bytes: bad R=%d", R);
-    *out = (size_t)num_sms() * packed_size(R) * sizeof(double);
+    *out = (size_t)num_sms() * kGramBlocks * packed_size(R) * sizeof(double);
     return FTL_OK;
 }
 
@@ -1372,29 +1451,23 @@ extern "C" int ftl_weighted_gram(const double *lhs, const int32_t *rowidx, const
     size_t need = 0;
     ftl_gram_workspace_bytes(R, &need);
     FTL_CHECK_ARG(ws_bytes >= need, "ftl_weighted_gram: workspace %zu < %zu bytes", ws_bytes, need);
-    const int nblk = num_sms();
     cudaStream_t st = (cudaStream_t)stream;
     const size_t smem = (size_t)(64 * R) * sizeof(double);
     const int P = packed_size(R);
-    const int threads = gram_threads(R);
-    const int ept = (P + threads - 1) / threads;
-    {
-        const void *fn = ept <= 1   ? (const void *)gram_partial_kernel<1>
-                         : ept <= 2 ? (const void *)gram_partial_kernel<2>
-                         : ept <= 4 ? (const void *)gram_partial_kernel<4>
-                                    : (const void *)gram_partial_kernel<9>;
-        const int arc = ensure_smem(fn, smem, "gram_partial_kernel");
-        if (arc) return arc;
-    }
-    double *part = (double *)workspace;
-    if (ept <= 1)
-        gram_partial_kernel<1><<<nblk, threads, smem, st>>>(lhs, rowidx, w, cnt, n_rows_dev, n_rows, R, part);
-    else if (ept <= 2)
-        gram_partial_kernel<2><<<nblk, threads, smem, st>>>(lhs, rowidx, w, cnt, n_rows_dev, n_rows, R, part);
-    else if (ept <= 4)
-        gram_partial_kernel<4><<<nblk, threads, smem, st>>>(lhs, rowidx, w, cnt, n_rows_dev, n_rows, R, part);
-    else
-        gram_partial_kernel<9><<<nblk, threads, smem, st>>>(lhs, rowidx, w, cnt, n_rows_dev, n_rows, R, part);
+    int ept, threads;
+    gram_shape(R, ept, threads);
+    const auto kernel = ept == 1   ? gram_partial_kernel<1>
+                        : ept == 2 ? gram_partial_kernel<2>
+                        : ept == 3 ? gram_partial_kernel<3>
+                        : ept == 5 ? gram_partial_kernel<5>
+                        : ept == 8 ? gram_partial_kernel<8>
+                                   : gram_partial_kernel<9>;
+    const int arc = ensure_smem((const void *)kernel, smem, "gram_partial_kernel");
+    if (arc) return arc;
+    int occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem) != cudaSuccess || occ < 1) occ = 1;
+    const int nblk = num_sms() * std::min(occ, kGramBlocks);
+    kernel<<<nblk, threads, smem, st>>>(lhs, rowidx, w, cnt, n_rows_dev, n_rows, R, (double *)workspace);
     gram_reduce_kernel<<<std::max(1, (P * 32 + 255) / 256), 256, 0, st>>>((const double *)workspace, nblk, R,
                                                                           gram_out);
     return check_launch("weighted gram kernels");
@@ -1437,18 +1510,14 @@ extern "C" int ftl_sparse_mttkrp(const uint64_t *sorted_keys, const uint32_t *so
 extern "C" int ftl_solve_rows(const double *B, const double *pinv, int64_t I, int R, double *U, void *stream) {
     FTL_CHECK_ARG(B && pinv && U, "ftl_solve_rows: null pointer");
     FTL_CHECK_ARG(R >= 1 && R <= FTL_MAX_RANK && I >= 1, "ftl_solve_rows: bad shape");
-    // R x R pinv plus one staged row per thread: 128 threads up to R = 64
-    // (96 KB), 64 threads above (196 KB at R = 128)
-    const int threads = R > 64 ? 64 : 128;
-    const size_t smem = (size_t)(R * R + threads * R) * sizeof(double);
-    FTL_CHECK_ARG(smem <= 227 * 1024, "ftl_solve_rows: R=%d too large", R);
-    {
-        const int arc = ensure_smem((const void *)solve_rows_kernel, smem, "solve_rows_kernel");
-        if (arc) return arc;
-    }
-    int blocks = (int)std::min<int64_t>((I + threads - 1) / threads, (int64_t)num_sms() * 8);
-    solve_rows_kernel<<<blocks, threads, smem, (cudaStream_t)stream>>>(B, pinv, I, R, U);
-    return check_launch("solve_rows_kernel");
+    return solve_rows(B, pinv, nullptr, nullptr, I, R, U, (cudaStream_t)stream);
+}
+
+extern "C" int ftl_solve_rows_at(const double *B, const double *pinv, const int32_t *rowidx, const int64_t *n_dev,
+                                 int64_t n_max, int R, double *U, void *stream) {
+    FTL_CHECK_ARG(B && pinv && U && rowidx && n_dev, "ftl_solve_rows_at: null pointer");
+    FTL_CHECK_ARG(R >= 1 && R <= FTL_MAX_RANK && n_max >= 1, "ftl_solve_rows_at: bad shape");
+    return solve_rows(B, pinv, rowidx, n_dev, n_max, R, U, (cudaStream_t)stream);
 }
 
 extern "C" int ftl_colnorm_workspace_bytes(int R, size_t *out) {
@@ -1468,7 +1537,7 @@ extern "C" int ftl_renormalize_columns(double *U, int64_t I, int R, double *norm
     const int threads = std::max(R, 1024 / R * R);
     cudaStream_t st = (cudaStream_t)stream;
     colsq_partial_kernel<<<nblk, threads, 0, st>>>(U, I, R, (double *)workspace);
-    colnorm_finish_kernel<<<1, 1024, 0, st>>>((const double *)workspace, nblk, R, norms_out);
+    colnorm_finish_kernel<<<(R + 3) / 4, 128, 0, st>>>((const double *)workspace, nblk, R, norms_out);
     if (apply) colscale_kernel<<<nblk * 2, threads, 0, st>>>(U, I, R, norms_out);
     return check_launch("renormalize kernels");
 }

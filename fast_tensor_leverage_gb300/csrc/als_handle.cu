@@ -367,8 +367,8 @@ extern "C" int ftl_als_update(ftl_als *A, int j, int renormalize, int update_sam
                                 stream)))
         return rc;
     if ((rc = ftl_pinv_square(A->gram, R, R, A->nuniq, 1e-11, A->pinv, A->vscr, stream))) return rc;
-    // U_j = MTTKRP pinv, with the J sampled rows multiplied by pinv first
-    if ((rc = ftl_solve_rows(A->h, A->pinv, J, R, A->hp, stream))) return rc;
+    // U_j = MTTKRP pinv, with the unique sampled rows multiplied by pinv first
+    if ((rc = ftl_solve_rows_at(A->h, A->pinv, A->urep, A->nuniq, J, R, A->hp, stream))) return rc;
     if ((rc = ftl_sparse_mttkrp_rows(X->rows[j], X->rkeys[j], X->rvals[j], X->nnz, A->ukeys, A->urep, A->ucnt,
                                      A->nuniq, J, J, A->w, A->hp, R, A->ws_mtt, A->nb_mtt, A->U[j], X->dims[j],
                                      stream)))

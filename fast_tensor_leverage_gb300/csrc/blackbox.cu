@@ -174,10 +174,11 @@ __global__ void chain_prod_kernel(BBGrams gp, int N, int Ra, int Rb, int exclude
     }
     red[threadIdx.x] = acc;
     __syncthreads();
-    if (threadIdx.x == 0 && out_sum) {
+    if (threadIdx.x < 32 && out_sum) {  // one warp, fixed order
         double s = 0.0;
-        for (int t = 0; t < (int)blockDim.x; ++t) s += red[t];
-        *out_sum = s;
+        for (int t = threadIdx.x; t < (int)blockDim.x; t += 32) s += red[t];
+        s = warp_sum(s);
+        if (threadIdx.x == 0) *out_sum = s;
     }
 }
 
@@ -413,12 +414,12 @@ extern "C" int ftl_lowrank_mttkrp_workspace_bytes(int Rr, int R, size_t *out) {
     return FTL_OK;
 }
 
-extern "C" int ftl_lowrank_sampled_mttkrp(const double *const *V, const double *sigma_rhs, int N, int Rr, int j,
-                                          const uint64_t *samples, int64_t J, const int32_t *urep,
-                                          const int32_t *ucnt, const int64_t *num_unique_dev, int64_t num_unique,
-                                          const double *w, const double *h, int R, void *workspace,
-                                          size_t ws_bytes, double *out, int64_t I_j, int64_t out_rows,
-                                          void *stream) {
+// pinv (R x R) given: (P^T L) pinv takes the place of P^T L.
+static int lowrank_mttkrp(const double *const *V, const double *sigma_rhs, int N, int Rr, int j,
+                          const uint64_t *samples, int64_t J, const int32_t *urep, const int32_t *ucnt,
+                          const int64_t *num_unique_dev, int64_t num_unique, const double *w, const double *h, int R,
+                          const double *pinv, void *workspace, size_t ws_bytes, double *out, int64_t I_j,
+                          int64_t out_rows, void *stream) {
     FTL_CHECK_ARG(V && samples && h && workspace && out, "ftl_lowrank_sampled_mttkrp: null pointer");
     FTL_CHECK_ARG(N >= 1 && N <= FTL_MAX_MODES && j >= 0 && j < N && Rr >= 1 && Rr <= FTL_MAX_RANK && R >= 1 &&
                       R <= FTL_MAX_RANK && I_j >= 1 && out_rows >= I_j && J >= 1,
@@ -441,9 +442,36 @@ extern "C" int ftl_lowrank_sampled_mttkrp(const double *const *V, const double *
     const size_t sm2 = (size_t)Rr * R * sizeof(double);
     rc = smem_attr((const void *)rows_times_small_kernel, sm2);
     if (rc) return rc;
+    if (pinv) {
+        const size_t sm3 = (size_t)R * R * sizeof(double);
+        rc = smem_attr((const void *)rows_times_small_kernel, std::max(sm2, sm3));
+        if (rc) return rc;
+        rows_times_small_kernel<<<std::max(1, (Rr * R + 255) / 256), 256, sm3, st>>>(M, Rr, R, pinv, R, partial, Rr);
+        M = partial;  // the block partials are summed
+    }
     int blocks = (int)std::min<int64_t>((out_rows * R + 255) / 256, (int64_t)nblk * 16);
     rows_times_small_kernel<<<std::max(blocks, 1), 256, sm2, st>>>(V[j], I_j, Rr, M, R, out, out_rows);
     return check_launch("low-rank sampled MTTKRP kernels");
+}
+
+extern "C" int ftl_lowrank_sampled_mttkrp(const double *const *V, const double *sigma_rhs, int N, int Rr, int j,
+                                          const uint64_t *samples, int64_t J, const int32_t *urep,
+                                          const int32_t *ucnt, const int64_t *num_unique_dev, int64_t num_unique,
+                                          const double *w, const double *h, int R, void *workspace,
+                                          size_t ws_bytes, double *out, int64_t I_j, int64_t out_rows,
+                                          void *stream) {
+    return lowrank_mttkrp(V, sigma_rhs, N, Rr, j, samples, J, urep, ucnt, num_unique_dev, num_unique, w, h, R, nullptr,
+                          workspace, ws_bytes, out, I_j, out_rows, stream);
+}
+
+extern "C" int ftl_lowrank_sampled_solve(const double *const *V, const double *sigma_rhs, int N, int Rr, int j,
+                                         const uint64_t *samples, int64_t J, const int32_t *urep,
+                                         const int32_t *ucnt, const int64_t *num_unique_dev, int64_t num_unique,
+                                         const double *w, const double *h, int R, const double *pinv, void *workspace,
+                                         size_t ws_bytes, double *out, int64_t I_j, int64_t out_rows, void *stream) {
+    FTL_CHECK_ARG(pinv, "ftl_lowrank_sampled_solve: pinv is NULL");
+    return lowrank_mttkrp(V, sigma_rhs, N, Rr, j, samples, J, urep, ucnt, num_unique_dev, num_unique, w, h, R, pinv,
+                          workspace, ws_bytes, out, I_j, out_rows, stream);
 }
 
 extern "C" int ftl_cross_gram_workspace_bytes(int Ra, int Rb, size_t *out) {

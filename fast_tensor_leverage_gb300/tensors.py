@@ -313,6 +313,14 @@ def _lr_sampled_mttkrp_dev(self, samples, J, urep, ucnt, nuniq, w, h, R, j, out,
                   urep, ucnt, nuniq, J, w, h, R, out, out_rows, stream)
 
 
+def _lr_sampled_solve_dev(self, samples, J, urep, ucnt, nuniq, w, h, pinv, R, j, out, out_rows, stream) -> None:
+    # the sampled MTTKRP times pinv, for a tensor without noise (its noise term has no low-rank middle)
+    nb = _lib.ws_bytes("lowrank_mttkrp", self.R, R)
+    ws = self._ws.get("lowrank_mttkrp", nb)
+    _lib.call("ftl_lowrank_sampled_solve", _ptrs(self.U_dev), self.sigma_dev.data_ptr(), self.N, self.R, j,
+              samples, J, urep, ucnt, nuniq, J, w, h, R, pinv, ws.data_ptr(), nb, out, self.dims[j], out_rows, stream)
+
+
 def _lr_execute_downsampled_mttkrp_py(self, samples, lhs, j: int, result) -> None:
     """result (I_j x R) = sum over the rows s of samples (J x N uint64) of
     fiber_s (x) lhs[s] (BlackBoxTensor::execute_downsampled_mttkrp,
@@ -354,6 +362,7 @@ LowRankTensor.evaluate_indices = _lr_evaluate_indices
 LowRankTensor.materialize_rhs = _lr_materialize_rhs
 LowRankTensor.execute_downsampled_mttkrp_py = _lr_execute_downsampled_mttkrp_py
 LowRankTensor._sampled_mttkrp_dev = _lr_sampled_mttkrp_dev
+LowRankTensor._sampled_solve_dev = _lr_sampled_solve_dev
 LowRankTensor._exact_mttkrp_dev = _lr_exact_mttkrp_dev
 
 

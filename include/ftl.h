@@ -322,6 +322,11 @@ int ftl_sparse_mttkrp_rows(const int32_t *row_idx, const uint64_t *row_keys,
 int ftl_solve_rows(const double *B_dev, const double *pinv_dev, int64_t I, int R, double *U_dev,
                    void *stream);
 
+/* ftl_solve_rows for the rows rowidx[u], u < *n_dev (<= n_max): the unique
+ * sampled rows of an ALS update, the only ones its MTTKRP reads. */
+int ftl_solve_rows_at(const double *B_dev, const double *pinv_dev, const int32_t *rowidx_dev,
+                      const int64_t *n_dev, int64_t n_max, int R, double *U_dev, void *stream);
+
 /* Handle form of the sparse tensor and of the randomized CP-ALS for hosts
  * that are not Python (SparseTensor + SortIdxLookup, sparse_tensor.hpp:46-77,
  * sort_lookup.hpp:33-60; ALS initialize_ds_als / execute_ds_als_update,
@@ -426,6 +431,13 @@ int ftl_lowrank_sampled_mttkrp(const double *const *V, const double *sigma_rhs, 
                                const int64_t *num_unique_dev, int64_t num_unique, const double *w,
                                const double *h, int R, void *workspace, size_t ws_bytes, double *out,
                                int64_t I_j, int64_t out_rows, void *stream);
+/* The same times pinv (R x R): out = V_j (P^T L) pinv, an ALS update's solve
+ * done on the Rr x R matrix in the middle instead of on the J sampled rows. */
+int ftl_lowrank_sampled_solve(const double *const *V, const double *sigma_rhs, int N, int Rr, int j,
+                              const uint64_t *samples, int64_t J, const int32_t *urep, const int32_t *ucnt,
+                              const int64_t *num_unique_dev, int64_t num_unique, const double *w,
+                              const double *h, int R, const double *pinv, void *workspace, size_t ws_bytes,
+                              double *out, int64_t I_j, int64_t out_rows, void *stream);
 /* Dense row-major tensor (FP64 or FP32, dims[N]): fiber = T[s_0, .., :, .., s_N-1]
  * (DenseTensor::materialize_rhs, cpp_ext/dense_tensor.hpp:38-59). */
 int ftl_dense_sampled_mttkrp(const void *T, int is_f32, const int64_t *dims, int N, int j,
