@@ -158,6 +158,8 @@ SIGNATURES = {
     "ftl_sparse_residual_terms": ([_P, _P, _I64, _INT, _P, _P, _INT, _P, ctypes.c_size_t, _P, _P], _INT),
     "ftl_sum_squares": ([_P, _I64, _P, ctypes.c_size_t, _P, _P], _INT),
     "ftl_sparse_exact_mttkrp": ([_P, _P, _I64, _INT, _INT, _P, _INT, _P, _I64, _P], _INT),
+    "ftl_sparse_residual_terms_scaled": ([_P, _P, _I64, _INT, _P, _P, _INT, _I64, _P, _INT, _P, ctypes.c_size_t, _P,
+                                         _P], _INT),
     "ftl_solve_rows_at": ([_P, _P, _P, _P, _I64, _INT, _P, _P], _INT),
     "ftl_sparse_exact_mttkrp_rows": ([_P, _P, _P, _I64, _INT, _P, _INT, _P, _INT, _P, _I64, _P], _INT),
     "ftl_gram_hadamard": ([_P, _INT, _INT, _INT, _P, _P, _P, _P, _P], _INT),

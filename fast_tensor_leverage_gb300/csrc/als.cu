@@ -1067,15 +1067,20 @@ __global__ void residual_partial_kernel(const uint32_t *__restrict__ idx, const 
 // row pointers stay in registers): R x N FP64 products per nonzero as lane
 // operations.  The warp-per-nonzero form above spends most of its FP64 issue
 // on the warp reduction of each nonzero, and the FP64 pipe (one warp
-// instruction per 16 cycles per SM) is what bounds this pass.
-template <int N>
+// instruction per 16 cycles per SM) is what bounds this pass.  SIG false: one
+// of the factors already carries sigma, N - 1 products and one multiply-add
+// are left of N + 1 operations per column (2.5e7 nonzeros, 3 modes, R = 25:
+// 3.62 -> 2.45 ms).
+template <int N, bool SIG>
 __global__ void residual_thread_kernel(const uint32_t *__restrict__ idx, const double *__restrict__ vals,
                                        int64_t nnz, FactorPtrs fp, const double *__restrict__ sigma, int R,
                                        double *__restrict__ partial) {
     __shared__ double sig[FTL_MAX_RANK];
     __shared__ double red[32];
-    for (int r = threadIdx.x; r < R; r += blockDim.x) sig[r] = sigma[r];
-    __syncthreads();
+    if (SIG) {
+        for (int r = threadIdx.x; r < R; r += blockDim.x) sig[r] = sigma[r];
+        __syncthreads();
+    }
     double acc = 0.0;
     for (int64_t z = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; z < nnz; z += (int64_t)gridDim.x * blockDim.x) {
         const double *row[N];
@@ -1083,10 +1088,12 @@ __global__ void residual_thread_kernel(const uint32_t *__restrict__ idx, const d
         for (int k = 0; k < N; ++k) row[k] = fp.U[k] + (int64_t)idx[z * N + k] * R;
         double m = 0.0;
         for (int r = 0; r < R; ++r) {
-            double p = sig[r];
+            double p = SIG ? sig[r] : row[0][r];
 #pragma unroll
-            for (int k = 0; k < N; ++k) p *= row[k][r];
-            m += p;
+            for (int k = SIG ? 0 : 1; k < N; ++k) {
+                if (k == N - 1) m = fma(p, row[k][r], m);
+                else p *= row[k][r];
+            }
         }
         const double v = vals[z];
         acc += v * v - 2.0 * m * v;
@@ -1099,6 +1106,16 @@ __global__ void residual_thread_kernel(const uint32_t *__restrict__ idx, const d
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
         partial[blockIdx.x] = t;
     }
+}
+
+// out[i][r] = U[i][r] s[r]
+__global__ void scale_columns_kernel(const double *__restrict__ U, int64_t total, int R, const double *__restrict__ s,
+                                     double *__restrict__ out) {
+    __shared__ double sh[FTL_MAX_RANK];
+    for (int r = threadIdx.x; r < R; r += blockDim.x) sh[r] = s[r];
+    __syncthreads();
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x)
+        out[e] = U[e] * sh[(uint64_t)e % (uint32_t)R];
 }
 
 // *out = sum of the n partials in a fixed order (lane-strided sums, then a
@@ -1548,6 +1565,38 @@ extern "C" int ftl_fit_workspace_bytes(size_t *out) {
     return FTL_OK;
 }
 
+template <int N, bool SIG>
+static int residual_threads(const uint32_t *idx, const double *vals, int64_t nnz, const FactorPtrs &fp,
+                            const double *sigma, int R, double *part, cudaStream_t st) {
+    // one wave of resident CTAs (equal work per CTA: a grid of a few waves plus
+    // a fraction leaves SMs idle at the end)
+    int nblk = num_sms() * 16, occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, residual_thread_kernel<N, SIG>, 256, 0) == cudaSuccess &&
+        occ >= 1)
+        nblk = num_sms() * std::min(occ, 16);
+    residual_thread_kernel<N, SIG><<<nblk, 256, 0, st>>>(idx, vals, nnz, fp, sigma, R, part);
+    return nblk;
+}
+
+template <bool SIG>
+static int residual_terms(const uint32_t *idx, const double *vals, int64_t nnz, int N, const double *const *U_dev,
+                          const double *sigma, int R, void *workspace, double *out, cudaStream_t st) {
+    FactorPtrs fp;
+    for (int k = 0; k < FTL_MAX_MODES; ++k) fp.U[k] = k < N ? U_dev[k] : nullptr;
+    double *part = (double *)workspace;
+    int nblk = num_sms() * 16;
+    switch (N) {
+        case 2: nblk = residual_threads<2, SIG>(idx, vals, nnz, fp, sigma, R, part, st); break;
+        case 3: nblk = residual_threads<3, SIG>(idx, vals, nnz, fp, sigma, R, part, st); break;
+        case 4: nblk = residual_threads<4, SIG>(idx, vals, nnz, fp, sigma, R, part, st); break;
+        case 5: nblk = residual_threads<5, SIG>(idx, vals, nnz, fp, sigma, R, part, st); break;
+        case 6: nblk = residual_threads<6, SIG>(idx, vals, nnz, fp, sigma, R, part, st); break;
+        default: residual_partial_kernel<<<nblk, 256, 0, st>>>(idx, vals, nnz, N, fp, sigma, R, part);
+    }
+    sum_kernel<<<1, 32, 0, st>>>(part, nblk, out);
+    return check_launch("residual kernels");
+}
+
 extern "C" int ftl_sparse_residual_terms(const uint32_t *idx, const double *vals, int64_t nnz, int N,
                                          const double *const *U_dev, const double *sigma, int R, void *workspace,
                                          size_t ws_bytes, double *out, void *stream) {
@@ -1556,31 +1605,25 @@ extern "C" int ftl_sparse_residual_terms(const uint32_t *idx, const double *vals
     size_t need = 0;
     ftl_fit_workspace_bytes(&need);
     FTL_CHECK_ARG(ws_bytes >= need, "ftl_sparse_residual_terms: workspace too small");
-    FactorPtrs fp;
-    for (int k = 0; k < FTL_MAX_MODES; ++k) fp.U[k] = k < N ? U_dev[k] : nullptr;
+    return residual_terms<true>(idx, vals, nnz, N, U_dev, sigma, R, workspace, out, (cudaStream_t)stream);
+}
+
+extern "C" int ftl_sparse_residual_terms_scaled(const uint32_t *idx, const double *vals, int64_t nnz, int N,
+                                                const double *const *U_dev, const double *sigma, int k,
+                                                int64_t k_rows, double *scaled, int R, void *workspace,
+                                                size_t ws_bytes, double *out, void *stream) {
+    FTL_CHECK_ARG(idx && vals && U_dev && sigma && scaled && workspace && out,
+                  "ftl_sparse_residual_terms_scaled: null pointer");
+    FTL_CHECK_ARG(N >= 2 && N <= 6 && R >= 1 && R <= FTL_MAX_RANK && k >= 0 && k < N && k_rows >= 1,
+                  "ftl_sparse_residual_terms_scaled: bad shape (2 to 6 modes)");
+    size_t need = 0;
+    ftl_fit_workspace_bytes(&need);
+    FTL_CHECK_ARG(ws_bytes >= need, "ftl_sparse_residual_terms_scaled: workspace too small");
     cudaStream_t st = (cudaStream_t)stream;
-    double *part = (double *)workspace;
-    // one wave of resident CTAs for the thread-per-nonzero forms (equal work
-    // per CTA: a grid of a few waves plus a fraction leaves SMs idle at the end)
-    int nblk = num_sms() * 16;
-    if (N >= 2 && N <= 6) {
-        const void *fn = N == 2 ? (const void *)residual_thread_kernel<2> : N == 3 ? (const void *)residual_thread_kernel<3>
-                       : N == 4 ? (const void *)residual_thread_kernel<4> : N == 5 ? (const void *)residual_thread_kernel<5>
-                                                                           : (const void *)residual_thread_kernel<6>;
-        int occ = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, 256, 0) == cudaSuccess && occ >= 1)
-            nblk = num_sms() * std::min(occ, 16);
-    }
-    switch (N) {
-        case 2: residual_thread_kernel<2><<<nblk, 256, 0, st>>>(idx, vals, nnz, fp, sigma, R, part); break;
-        case 3: residual_thread_kernel<3><<<nblk, 256, 0, st>>>(idx, vals, nnz, fp, sigma, R, part); break;
-        case 4: residual_thread_kernel<4><<<nblk, 256, 0, st>>>(idx, vals, nnz, fp, sigma, R, part); break;
-        case 5: residual_thread_kernel<5><<<nblk, 256, 0, st>>>(idx, vals, nnz, fp, sigma, R, part); break;
-        case 6: residual_thread_kernel<6><<<nblk, 256, 0, st>>>(idx, vals, nnz, fp, sigma, R, part); break;
-        default: residual_partial_kernel<<<nblk, 256, 0, st>>>(idx, vals, nnz, N, fp, sigma, R, part);
-    }
-    sum_kernel<<<1, 32, 0, st>>>((const double *)workspace, nblk, out);
-    return check_launch("residual kernels");
+    scale_columns_kernel<<<grid_for(k_rows * R), 256, 0, st>>>(U_dev[k], k_rows * R, R, sigma, scaled);
+    const double *U[FTL_MAX_MODES];
+    for (int m = 0; m < N; ++m) U[m] = m == k ? scaled : U_dev[m];
+    return residual_terms<false>(idx, vals, nnz, N, U, nullptr, R, workspace, out, st);
 }
 
 extern "C" int ftl_sum_squares(const double *v, int64_t n, void *workspace, size_t ws_bytes, double *out,

@@ -559,8 +559,17 @@ class SparseTensor:
         Ud = self._factor_dev(U_list, R)
         nb = _lib.ws_bytes("fit")
         terms = torch.empty(2, dtype=torch.float64, device=self.device)
-        _lib.call("ftl_sparse_residual_terms", self.idx_dev.data_ptr(), self.vals_dev.data_ptr(), self.nnz, self.N,
-                  _ptrs(Ud), sig.data_ptr(), R, self._ws.get("fit", nb).data_ptr(), nb, terms[0:1].data_ptr(), st)
+        k = min(range(self.N), key=lambda m: Ud[m].shape[0])
+        if 2 <= self.N <= 6 and 2 * Ud[k].shape[0] <= self.nnz:
+            # sigma goes into the factor with the fewest rows: cheaper than a product per nonzero
+            scaled = torch.empty_like(Ud[k])
+            _lib.call("ftl_sparse_residual_terms_scaled", self.idx_dev.data_ptr(), self.vals_dev.data_ptr(), self.nnz,
+                      self.N, _ptrs(Ud), sig.data_ptr(), k, Ud[k].shape[0], scaled.data_ptr(), R,
+                      self._ws.get("fit", nb).data_ptr(), nb, terms[0:1].data_ptr(), st)
+        else:
+            _lib.call("ftl_sparse_residual_terms", self.idx_dev.data_ptr(), self.vals_dev.data_ptr(), self.nnz,
+                      self.N, _ptrs(Ud), sig.data_ptr(), R, self._ws.get("fit", nb).data_ptr(), nb,
+                      terms[0:1].data_ptr(), st)
         G = [factor_gram(u, self._ws, st) for u in Ud]
         _lib.call("ftl_gram_hadamard", _ptrs(G), self.N, R, -1, sig.data_ptr(), sig.data_ptr(), None,
                   terms[1:2].data_ptr(), st)

@@ -382,6 +382,14 @@ int ftl_fit_workspace_bytes(size_t *out);
 int ftl_sparse_residual_terms(const uint32_t *idx_dev, const double *vals_dev, int64_t nnz, int N,
                               const double *const *U_dev, const double *sigma_dev, int R,
                               void *workspace, size_t ws_bytes, double *out_dev, void *stream);
+/* The same for 2 to 6 modes with sigma carried by factor k (k_rows rows):
+ * scaled (k_rows x R) receives U_k times sigma, and the pass over the nonzeros
+ * does one product less per column. */
+int ftl_sparse_residual_terms_scaled(const uint32_t *idx_dev, const double *vals_dev, int64_t nnz, int N,
+                                     const double *const *U_dev, const double *sigma_dev, int k,
+                                     int64_t k_rows, double *scaled_dev, int R, void *workspace,
+                                     size_t ws_bytes, double *out_dev, void *stream);
+
 /* *out = sum of v_i^2 (SparseTensor's normsq, cpp_ext/sparse_tensor.hpp:70-74). */
 int ftl_sum_squares(const double *v_dev, int64_t n, void *workspace, size_t ws_bytes,
                     double *out_dev, void *stream);

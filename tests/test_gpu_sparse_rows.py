@@ -59,3 +59,22 @@ def test_range_finder_rows(ftl, R):
         _lib.call("ftl_sparse_rrf", rrows.data_ptr(), rkeys.data_ptr(), rvals.data_ptr(), sp.nnz, R, seed, j,
                   out.data_ptr(), dims[j], torch.cuda.current_stream().cuda_stream)
         np.testing.assert_allclose(out.cpu().numpy(), U[j], rtol=0, atol=1e-5 * max(1.0, np.abs(U[j]).max()))
+
+
+@pytest.mark.parametrize("R", [1, 8, 25, 33, 128])
+@pytest.mark.parametrize("dims,nnz", [([700, 30, 40], 5000), ([60, 80], 257), ([5, 300, 7, 11], 3000),
+                                      ([3, 4, 2, 3, 5, 4], 700), ([2, 3, 2, 3, 2, 3, 4], 500), ([900, 800, 700], 100)])
+def test_residual_terms(ftl, dims, nnz, R):
+    rng, idx, vals = tensor(dims, nnz, R + nnz)
+    sp = ftl.SparseTensor(idx, vals, "sort", dims=dims)
+    U = [rng.normal(size=(d, R)) for d in dims]
+    s = rng.random(R) + 0.5
+    m = np.ones((idx.shape[0], R)) * s
+    G = np.outer(s, s)
+    for k in range(len(dims)):
+        m = m * U[k][idx[:, k]]
+        G = G * (U[k].T @ U[k])
+    terms = sp.residual_terms_async(torch.from_numpy(s).cuda(), [torch.from_numpy(u).cuda() for u in U]).cpu().numpy()
+    first = vals ** 2 - 2.0 * vals * m.sum(axis=1)
+    assert abs(terms[0] - first.sum()) <= 1e-12 * max(1.0, (vals ** 2 + 2.0 * np.abs(vals) * np.abs(m).sum(axis=1)).sum())
+    assert abs(terms[1] - G.sum()) <= 1e-12 * np.abs(G).sum()
