@@ -468,10 +468,14 @@ __device__ __forceinline__ void split_bits53(uint64_t B, float &dh, float &dl) {
     dl = (float)(uint32_t)(B & 0x1fffffffu) * 1.1102230246251565e-16f;  // 2^-53
 }
 
+// tab, tl_levels: forms of the root and of the left children on the first
+// tl_levels levels read from a mass table (draw_params.cuh) instead of
+// evaluated.
 template <int RMAX, class QF>
 __device__ __forceinline__ int64_t descend_df(const float *__restrict__ G, int S, const DGeom &g, float dh,
                                               float dl, const QF &qf, int lane, float &frac,
-                                              const double *U = nullptr, int R = 0, float *mroot = nullptr) {
+                                              const double *U = nullptr, int R = 0, float *mroot = nullptr,
+                                              const float *tab = nullptr, int tab_levels = 0) {
     int64_t c = 0;
     if (is_leaf(g, 0)) {  // single-leaf tree: the leaf fraction is the draw
         frac = fminf(dh + dl, 1.0f);
@@ -480,7 +484,10 @@ __device__ __forceinline__ int64_t descend_df(const float *__restrict__ G, int S
     }
     prefetch_next(G, S, g, 0, U, R, lane);
     float mP, mL0;
-    if (FTL_DESC_EVAL2) {
+    if (tab_levels > 0) {
+        mP = __ldg(tab);
+        mL0 = __ldg(tab + 1);
+    } else if (FTL_DESC_EVAL2) {
         qf.eval2(G, G + S, lane, mP, mL0);
     } else {
         mP = qf.eval(G, lane);
@@ -505,6 +512,8 @@ __device__ __forceinline__ int64_t descend_df(const float *__restrict__ G, int S
         float mL;
         if (lvl == 0) {
             mL = mL0;
+        } else if (lvl < tab_levels) {
+            mL = __ldg(tab + 1 + cu);
         } else {
             prefetch_next(G, S, g, (int64_t)cu, U, R, lane);
             mL = qf.eval(G + (size_t)(2u * cu + 1u) * (size_t)S, lane);
@@ -529,10 +538,10 @@ template <int RMAX, class QF>
 __device__ __forceinline__ int64_t descend(const float *__restrict__ G, int S, const DGeom &g,
                                            double draw, const QF &qf, int lane,
                                            float &frac, const double *U = nullptr, int R = 0,
-                                           float *mroot = nullptr) {
+                                           float *mroot = nullptr, const float *tab = nullptr, int tab_levels = 0) {
     float dh, dl;
     split_df(draw, dh, dl);
-    return descend_df<RMAX, QF>(G, S, g, dh, dl, qf, lane, frac, U, R, mroot);
+    return descend_df<RMAX, QF>(G, S, g, dh, dl, qf, lane, frac, U, R, mroot, tab, tab_levels);
 }
 
 // The FP32 descent above carries the mass of a right child as parent - left

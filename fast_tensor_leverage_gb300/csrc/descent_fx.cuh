@@ -255,10 +255,12 @@ struct FxLeaf {
 };
 
 // The descent of descent.cuh's FP64 `descend` for uniform D 2^-53; false when
-// a decision is closer than the error bound.
+// a decision is closer than the error bound.  The forms of the root and of the
+// first tab_levels levels come from a mass table (tab_levels = -1: none).
 template <int RMAX, int TW, int FR>
 __device__ __forceinline__ bool fx_descend(FxTeam<RMAX, TW> &tm, const double *__restrict__ G, int S, const DGeom &g,
-                                           uint64_t D, const FxScale &sc, FxLeaf &out) {
+                                           uint64_t D, const FxScale &sc, FxLeaf &out, const int64_t *tab,
+                                           int tab_levels) {
     const int64_t E = (int64_t)kFxErr * TW * fx_flushes(tm);
     const uint32_t ncount = (uint32_t)g.node_count;
     const int lf = (int)g.lfill_level;
@@ -267,7 +269,9 @@ __device__ __forceinline__ bool fx_descend(FxTeam<RMAX, TW> &tm, const double *_
     const double *node = G;
 #pragma unroll 1
     for (int lvl = -1;; ++lvl) {
-        const int64_t f = fx_eval<RMAX, TW, FR>(tm, node, sc);
+        int64_t f;
+        if (lvl < tab_levels) f = __ldg((const long long *)tab + (lvl < 0 ? 0 : 1 + c));
+        else f = fx_eval<RMAX, TW, FR>(tm, node, sc);
         if (lvl < 0) {
             if (f <= 16 * E) return false;
             m = f;

@@ -86,6 +86,7 @@ __device__ __forceinline__ void draw_sample(const DrawParams &p, int64_t i, Draw
         double x[XPL];
 #pragma unroll
         for (int q = 0; q < XPL; ++q) x[q] = h[q];
+        int64_t comp = 0;  // eigen component
 #pragma unroll 1
         for (int phase = 0; phase < 2; ++phase) {
             const T *G = phase == 0 ? (const T *)p.eig_G + k * eig_stride : (const T *)p.gram_G[k];
@@ -95,14 +96,24 @@ __device__ __forceinline__ void draw_sample(const DrawParams &p, int64_t i, Draw
             stage_query<RMAX, T>(x, R, xd, xT, lane);
             qf.setup(xT, pairs, lane);
             T frac, mroot = T(1);
+            const T *tab = nullptr;
+            int tab_levels = 0;
+            if (sizeof(T) == 4 && !CAREFUL && p.table != nullptr && k == p.tab_mode) {
+                tab = (const T *)p.table + (phase == 0 ? 0 : kTabEig + comp * kTabNodes);
+                tab_levels = phase == 0 ? kTabLevels : p.tab_levels;
+            }
             const double u = get_draw(p, (int64_t)(phase * p.N + k) * p.J + i);
             int64_t c;
             if constexpr (CAREFUL && sizeof(T) == 4)
                 c = descend_careful<RMAX>(G, p.S, g, u, qf, lane, frac);
+            else if constexpr (sizeof(T) == 4)
+                c = descend<RMAX>(G, p.S, g, u, qf, lane, frac, (phase == 1 && g.F > 1) ? Uk : nullptr, R, &mroot, tab,
+                                  tab_levels);
             else
                 c = descend<RMAX>(G, p.S, g, u, qf, lane, frac, (phase == 1 && g.F > 1) ? Uk : nullptr, R, &mroot);
             if (phase == 0) {
-                const double *Wr = p.M + (size_t)p.offset[k] * RR + (size_t)leaf_index(g, c) * R;
+                comp = leaf_index(g, c);
+                const double *Wr = p.M + (size_t)p.offset[k] * RR + (size_t)comp * R;
 #pragma unroll
                 for (int q = 0; q < XPL; ++q) {
                     int col = lane + 32 * q;
@@ -301,6 +312,59 @@ __global__ void __launch_bounds__(D32Shape<NC, SW>::WARPS * 32, D32Shape<NC, SW>
     const int warp = threadIdx.x >> 5;
     for (int64_t i0 = ((int64_t)blockIdx.x * WARPS + warp) * NC; i0 < p.J; i0 += (int64_t)gridDim.x * WARPS * NC)
         draw_samples_d32<S32, NC, SW>(p, i0, threadIdx.x & 31, SW ? d32_slots + warp * NC * kDiag32Stride : nullptr);
+}
+
+// Mass table of the first sampled mode (draw_params.cuh): a warp stages one
+// query -- component u's W[u], or h = 1 for the eigen tree (item R) -- and
+// evaluates kTabRun nodes with it, by the code the descents use.
+constexpr int kTabRun = 16;
+
+// Warp item -> query number (R: the eigen tree), first entry and end.
+__device__ __forceinline__ bool table_item(const DrawParams &p, int64_t item, int &u, int &t0, int &t1) {
+    const int runs = ((1 << p.tab_levels) + kTabRun - 1) / kTabRun, eruns = (p.R + kTabRun - 1) / kTabRun;
+    if (item < eruns) {
+        u = p.R;
+        t0 = (int)item * kTabRun;
+        t1 = min(p.R, t0 + kTabRun);  // root and the left children of R - 1 internal nodes
+        return true;
+    }
+    item -= eruns;
+    if (p.tab_levels == 0 || item >= (int64_t)runs * p.R) return false;
+    u = (int)(item / runs);
+    t0 = (int)(item % runs) * kTabRun;
+    t1 = min(1 << p.tab_levels, t0 + kTabRun);
+    return true;
+}
+
+static int64_t table_items(const DrawParams &p) {
+    return (p.R + kTabRun - 1) / kTabRun +
+           (p.tab_levels ? (int64_t)(((1 << p.tab_levels) + kTabRun - 1) / kTabRun) * p.R : 0);
+}
+
+template <int RMAX>
+__global__ void __launch_bounds__(Blk<RMAX, float>::WARPS * 32) krp_table_kernel(DrawParams p) {
+    constexpr int XPL = Shape<RMAX>::XPL;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    DrawWarp<RMAX, float, false> dw;
+    setup_draw_warp<RMAX, float, false>(dw, smem_raw, p.R, p.P, p.S);
+    const int lane = dw.lane, R = p.R, k = p.tab_mode;
+    int u, t0, t1;
+    if (!table_item(p, (int64_t)blockIdx.x * Blk<RMAX, float>::WARPS + (threadIdx.x >> 5), u, t0, t1)) return;
+    double x[XPL];
+#pragma unroll
+    for (int q = 0; q < XPL; ++q) {
+        const int col = lane + 32 * q;
+        x[q] = 1.0;
+        if (u < R) x[q] = col < R ? p.M[(size_t)p.offset[k] * R * R + (size_t)u * R + col] : 0.0;
+    }
+    stage_query<RMAX, float>(x, R, dw.xd, dw.xT, lane);
+    dw.qf.setup(dw.xT, dw.pairs, lane);
+    const float *G = u < R ? (const float *)p.gram_G[k] : (const float *)p.eig_G + (size_t)k * (2 * R - 1) * p.S;
+    float *tab = (float *)p.table + (u < R ? kTabEig + (size_t)u * kTabNodes : 0);
+    for (int t = t0; t < t1; ++t) {
+        const float m = dw.qf.eval(G + (size_t)(t == 0 ? 0 : 2 * t - 1) * p.S, lane);
+        if (lane == 0) tab[t] = m;
+    }
 }
 
 // Packed draw: the samples of up to FTL_MAX_PACK requests of the same rank
@@ -556,6 +620,18 @@ static int launch_d32(const DrawParams &p, cudaStream_t st) {
     return FTL_OK;
 }
 
+template <int RMAX>
+static int launch_table(const DrawParams &p, cudaStream_t st) {
+    if (p.table == nullptr) return FTL_OK;
+    const int64_t items = table_items(p);
+    const int warps = Blk<RMAX, float>::WARPS;
+    const size_t smem = desc_smem<RMAX, float, false>();
+    const int arc = ensure_smem((const void *)krp_table_kernel<RMAX>, smem, "krp_table_kernel");
+    if (arc) return arc;
+    krp_table_kernel<RMAX><<<(unsigned)((items + warps - 1) / warps), warps * 32, smem, st>>>(p);
+    return check_launch("krp_table_kernel");
+}
+
 template <int RMAX, bool S32, bool DIAG>
 static int launch_draw(const DrawParams &p, cudaStream_t st) {
     using T = float;
@@ -573,6 +649,8 @@ static int launch_draw(const DrawParams &p, cudaStream_t st) {
         }
         if (lrc) return lrc;
     } else {
+        const int trc = launch_table<RMAX>(p, st);
+        if (trc) return trc;
         const int arc = ensure_smem((const void *)krp_draw_kernel<RMAX, T, S32>, smem, "krp_draw_kernel");
         if (arc) return arc;
         int64_t blocks = (p.J + warps - 1) / warps;
@@ -704,7 +782,7 @@ extern "C" int ftl_krp_plan_sizes(int N, int R, int prec, size_t *eig_bytes, siz
     FTL_CHECK_ARG(valid_prec(prec), "ftl_krp_plan_sizes: bad precision");
     const int esize = prec_bytes(prec);
     if (eig_bytes) *eig_bytes = (size_t)N * (2 * R - 1) * node_stride(R, esize) * esize;
-    if (M_bytes) *M_bytes = (cm_pinv64_offset(N, R) + node_stride(R, 8)) * sizeof(double);
+    if (M_bytes) *M_bytes = cm_table_offset(N, R) * sizeof(double) + table_bytes(R, esize);
     if (lambda_bytes) *lambda_bytes = (size_t)(N + 1) * R * sizeof(double);
     if (pinv32_bytes) *pinv32_bytes = (size_t)node_stride(R, 4) * sizeof(float);
     return FTL_OK;
@@ -723,17 +801,34 @@ extern "C" int ftl_krp_compute_m(const ftl_krp_plan *plan, uint32_t j, void *str
 static void fill_draw_params(DrawParams &p, const ftl_krp_plan *plan, uint32_t j, uint64_t *samples, double *h,
                              double *weights, const double *draws, uint64_t seed, uint64_t ctr);
 
-extern "C" int ftl_krp_sample(const ftl_krp_plan *plan, uint32_t j, uint64_t *samples, double *h,
-                              double *weights, const double *draws, uint64_t seed, uint64_t ctr,
-                              void *stream) {
+// table: the plan's M holds room for the mass table (ftl_krp_plan_sizes).
+static int krp_sample(const ftl_krp_plan *plan, uint32_t j, uint64_t *samples, double *h, double *weights,
+                      const double *draws, uint64_t seed, uint64_t ctr, bool table, void *stream) {
     int rc = validate_plan(plan);
     if (rc) return rc;
     FTL_CHECK_ARG(samples != nullptr, "ftl_krp_sample: samples is NULL");
     DrawParams p;
     fill_draw_params(p, plan, j, samples, h, weights, draws, seed, ctr);
+    if (table) {
+        p.tab_mode = p.j == 0 ? 1 : 0;
+        // wrapped-diagonal trees: their upper levels come from L1 at 17 values
+        // per lane, and a table measured 2% either way (N = 3, I = 2^23, R = 32:
+        // 787 -> 769 us; an ALS update at R = 25: 1.93 -> 1.98 ms)
+        const bool diag = plan->prec == FTL_PREC_FP32 && node_layout(plan->R, 4) == FTL_LAYOUT_DIAG32;
+        if (p.tab_mode < p.N && !diag) {
+            p.tab_levels = table_levels(p.gram[p.tab_mode], p.R, plan->J);
+            if (p.tab_levels) p.table = plan->M + cm_table_offset(p.N, p.R);
+        }
+    }
     cudaStream_t st = (cudaStream_t)stream;
     if (plan->prec == FTL_PREC_FP64) return launch_draw_fx(p, st);
     return dispatch_draw_f32(p, st);
+}
+
+extern "C" int ftl_krp_sample(const ftl_krp_plan *plan, uint32_t j, uint64_t *samples, double *h,
+                              double *weights, const double *draws, uint64_t seed, uint64_t ctr,
+                              void *stream) {
+    return krp_sample(plan, j, samples, h, weights, draws, seed, ctr, true, stream);
 }
 
 static void fill_draw_params(DrawParams &p, const ftl_krp_plan *plan, uint32_t j, uint64_t *samples, double *h,
@@ -769,6 +864,8 @@ static void fill_draw_params(DrawParams &p, const ftl_krp_plan *plan, uint32_t j
     p.draws = draws;
     p.seed = seed;
     p.ctr = ctr;
+    p.table = nullptr;
+    p.tab_mode = p.tab_levels = 0;
 }
 
 static int sample_packed(const ftl_krp_plan *const *plans, int n, const uint32_t *js, uint64_t *const *samples,
@@ -851,6 +948,17 @@ extern "C" int ftl_krp_draw(const ftl_krp_plan *plan, uint32_t j, uint64_t *samp
     if (rc) return rc;
     return ftl_krp_sample(plan, j, samples, h, weights, draws, seed, ctr, stream);
 }
+
+namespace ftl {
+// The static draw's plan (krp_draw_static.cu): M without room for the table.
+size_t static_M_bytes(int N, int R) { return (cm_pinv64_offset(N, R) + node_stride(R, 8)) * sizeof(double); }
+int static_draw(const ftl_krp_plan *plan, uint32_t j, uint64_t *samples, double *h, double *weights,
+                const double *draws, uint64_t seed, uint64_t ctr, void *stream) {
+    int rc = ftl_krp_compute_m(plan, j, stream);
+    if (rc) return rc;
+    return krp_sample(plan, j, samples, h, weights, draws, seed, ctr, false, stream);
+}
+}  // namespace ftl
 
 extern "C" int ftl_tree_sample(const void *G, int prec, const double *U, int64_t n, int R, int64_t F,
                                double *h, const double *scaled_h, uint64_t *samples,

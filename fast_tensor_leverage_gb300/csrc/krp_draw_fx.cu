@@ -96,22 +96,18 @@ __device__ __noinline__ int64_t fx_redo(const DrawParams &p, const double *G, co
     return leaf_scan<RMAX, double, double>(U, p.R, g, c, frac, lane_query<RMAX, double>(xd, p.R, lane), lane, empty);
 }
 
-template <int RMAX, int FR>
-__global__ void __launch_bounds__(FxShape<RMAX>::THREADS, FxShape<RMAX>::MINB) krp_draw_fx_kernel(DrawParams p) {
+// The block's pair table and root exponents (eg: [eigen trees, Gram trees][N]),
+// and this thread's team.
+template <int RMAX>
+__device__ __forceinline__ void fx_setup(const DrawParams &p, unsigned char *smem, FxTeam<RMAX, FxShape<RMAX>::TW> &tm) {
     using Sh = FxShape<RMAX>;
     constexpr int TW = Sh::TW, TEAMS = Sh::TEAMS;
-    constexpr int XPL = Shape<RMAX>::XPL;
-    using Team = FxTeam<RMAX, TW>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
     const int R = p.R, N = p.N, lane = threadIdx.x & 31;
-    const size_t RR = (size_t)R * R;
     const size_t eig_stride = (size_t)(2 * R - 1) * p.S;
-    int *eg = (int *)smem_raw;  // largest diagonal exponent of the roots: [eigen trees, Gram trees][N]
-    int64_t *answer = (int64_t *)(smem_raw + 2 * FTL_MAX_MODES * sizeof(int));  // TW > 1: a redo's result
+    int *eg = (int *)smem;
     const FxSmem<RMAX> lay(R);
-    uint16_t *pairs = (uint16_t *)(smem_raw + kFxHead);
-    unsigned char *base = smem_raw + fx_head(R) + (threadIdx.x / (32 * TW)) * lay.team;
-    Team tm;
+    uint16_t *pairs = (uint16_t *)(smem + kFxHead);
+    unsigned char *base = smem + fx_head(R) + (threadIdx.x / (32 * TW)) * lay.team;
     tm.slot = (float4 *)(base + lay.slot);
     tm.xd = (double *)(base + lay.xd);
     tm.xs = (float2 *)(base + lay.xs);
@@ -139,6 +135,70 @@ __global__ void __launch_bounds__(FxShape<RMAX>::THREADS, FxShape<RMAX>::MINB) k
         if (lane == 0) eg[k] = (int)e;
     }
     __syncthreads();
+}
+
+// Mass table of the first sampled mode (draw_params.cuh): a team stages one
+// query -- component u's W[u], or h = 1 for the eigen tree -- and evaluates a
+// run of nodes with it.  A query or tree outside the scaling's range gives
+// zeros, which the descents leave to the FP64 code.
+constexpr int kFxTabRun = 16;
+
+static __host__ __device__ int64_t fx_table_items(const DrawParams &p) {
+    return (p.R + kFxTabRun - 1) / kFxTabRun +
+           (int64_t)(((1 << p.tab_levels) + kFxTabRun - 1) / kFxTabRun) * p.R;
+}
+
+template <int RMAX, int FR>
+__global__ void __launch_bounds__(FxShape<RMAX>::THREADS, FxShape<RMAX>::MINB) krp_table_fx_kernel(DrawParams p) {
+    using Sh = FxShape<RMAX>;
+    constexpr int TW = Sh::TW, TEAMS = Sh::TEAMS;
+    constexpr int XPL = Shape<RMAX>::XPL;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    FxTeam<RMAX, TW> tm;
+    fx_setup<RMAX>(p, smem_raw, tm);
+    const int *eg = (const int *)smem_raw;
+    const int R = p.R, lane = threadIdx.x & 31, k = p.tab_mode;
+    const int runs = ((1 << p.tab_levels) + kFxTabRun - 1) / kFxTabRun, eruns = (R + kFxTabRun - 1) / kFxTabRun;
+    const int64_t items = fx_table_items(p);
+    for (int64_t it = (int64_t)blockIdx.x * TEAMS + threadIdx.x / (32 * TW); it < items;
+         it += (int64_t)gridDim.x * TEAMS) {
+        const bool gram = it >= eruns;
+        const int u = gram ? (int)((it - eruns) / runs) : 0;
+        const int t0 = (gram ? (int)((it - eruns) % runs) : (int)it) * kFxTabRun;
+        const int t1 = min(gram ? 1 << p.tab_levels : R, t0 + kFxTabRun);
+        double x[XPL];
+#pragma unroll
+        for (int q = 0; q < XPL; ++q) {
+            const int col = lane + 32 * q;
+            x[q] = 0.0;
+            if (col < R) x[q] = gram ? p.M[(size_t)p.offset[k] * R * R + (size_t)u * R + col] : 1.0;
+        }
+        FxScale sc;
+        const bool ok = fx_stage(tm, x, R, eg[(gram ? p.N : 0) + k], sc);
+        const double *G = gram ? (const double *)p.gram_G[k] : (const double *)p.eig_G + (size_t)k * (2 * R - 1) * p.S;
+        int64_t *tab = (int64_t *)p.table + (gram ? kTabEig + (size_t)u * kTabNodes : 0);
+        for (int t = t0; t < t1; ++t) {
+            int64_t m = 0;
+            if (ok) m = fx_eval<RMAX, TW, FR>(tm, G + (size_t)(t == 0 ? 0 : 2 * t - 1) * p.S, sc);
+            if (tm.tid == 0) tab[t] = m;
+        }
+    }
+}
+
+template <int RMAX, int FR>
+__global__ void __launch_bounds__(FxShape<RMAX>::THREADS, FxShape<RMAX>::MINB) krp_draw_fx_kernel(DrawParams p) {
+    using Sh = FxShape<RMAX>;
+    constexpr int TW = Sh::TW, TEAMS = Sh::TEAMS;
+    constexpr int XPL = Shape<RMAX>::XPL;
+    using Team = FxTeam<RMAX, TW>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int R = p.R, N = p.N, lane = threadIdx.x & 31;
+    const size_t RR = (size_t)R * R;
+    const size_t eig_stride = (size_t)(2 * R - 1) * p.S;
+    const int *eg = (const int *)smem_raw;
+    int64_t *answer = (int64_t *)(smem_raw + 2 * FTL_MAX_MODES * sizeof(int));  // TW > 1: a redo's result
+    Team tm;
+    fx_setup<RMAX>(p, smem_raw, tm);
 
     const int64_t teams = (int64_t)gridDim.x * TEAMS;
 #pragma unroll 1
@@ -166,6 +226,7 @@ __global__ void __launch_bounds__(FxShape<RMAX>::THREADS, FxShape<RMAX>::MINB) k
             double x[XPL];
 #pragma unroll
             for (int q = 0; q < XPL; ++q) x[q] = lane + 32 * q < R ? h[q] : 0.0;
+            int64_t comp = 0;  // eigen component
 #pragma unroll 1
             for (int phase = 0; phase < 2; ++phase) {
                 const double *G = phase == 0 ? (const double *)p.eig_G + k * eig_stride : (const double *)p.gram_G[k];
@@ -174,7 +235,16 @@ __global__ void __launch_bounds__(FxShape<RMAX>::THREADS, FxShape<RMAX>::MINB) k
                 const uint64_t Dk = __shfl_sync(0xffffffffu, D, l);
                 FxScale sc;
                 FxLeaf lf;
-                bool ok = fx_stage(tm, x, R, eg[l], sc) && ((dmask >> l) & 1u);
+                // the first sampled mode: eigen component and upper Gram levels from the mass table
+                const bool tabled = p.table != nullptr && k == p.tab_mode;
+                const int64_t *tab = nullptr;
+                int tab_levels = -1;
+                if (tabled) {
+                    tab = (const int64_t *)p.table + (phase == 0 ? 0 : kTabEig + comp * kTabNodes);
+                    tab_levels = phase == 0 ? kTabLevels : p.tab_levels;
+                }
+                const bool staged = !tabled || phase == 1;
+                bool ok = (!staged || fx_stage(tm, x, R, eg[l], sc)) && ((dmask >> l) & 1u);
                 int64_t t = 0;
                 if (ok) {
                     if (is_leaf(g, 0)) {  // the leaf fraction is the draw
@@ -183,7 +253,7 @@ __global__ void __launch_bounds__(FxShape<RMAX>::THREADS, FxShape<RMAX>::MINB) k
                         lf.m = (int64_t)1 << 53;
                         lf.tol = lf.mtol = 1;
                     } else {
-                        ok = fx_descend<RMAX, TW, FR>(tm, G, p.S, g, Dk, sc, lf);
+                        ok = fx_descend<RMAX, TW, FR>(tm, G, p.S, g, Dk, sc, lf, tab, tab_levels);
                     }
                 }
                 if (ok) {
@@ -194,6 +264,7 @@ __global__ void __launch_bounds__(FxShape<RMAX>::THREADS, FxShape<RMAX>::MINB) k
                 }
                 if (!ok) {
                     const double u = get_draw(p, (int64_t)l * p.J + i);
+                    if (!staged) fx_stage(tm, x, R, eg[l], sc);
                     Team::sync();
                     if (TW == 1 || tm.tid < 32) {
                         t = fx_redo<RMAX>(p, G, g, p.U[k], (double *)tm.slot, tm.xd, tm.pairs, u, phase == 1, lane);
@@ -204,6 +275,7 @@ __global__ void __launch_bounds__(FxShape<RMAX>::THREADS, FxShape<RMAX>::MINB) k
                     Team::sync();
                 }
                 if (phase == 0) {
+                    comp = t;
                     const double *Wr = p.M + (size_t)p.offset[k] * RR + (size_t)t * R;
 #pragma unroll
                     for (int q = 0; q < XPL; ++q) {
@@ -257,6 +329,15 @@ static int launch_fx(const DrawParams &p, cudaStream_t st) {
     int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, Sh::THREADS, smem) != cudaSuccess || occ < 1)
         occ = 1;
+    if (p.table) {
+        const auto table = krp_table_fx_kernel<RMAX, FR>;
+        rc = ensure_smem((const void *)table, smem, "krp_table_fx_kernel");
+        if (rc) return rc;
+        const int64_t tneed = (fx_table_items(p) + Sh::TEAMS - 1) / Sh::TEAMS;
+        table<<<(int)std::min<int64_t>(tneed, (int64_t)num_sms() * occ), Sh::THREADS, smem, st>>>(p);
+        rc = check_launch("krp_table_fx_kernel");
+        if (rc) return rc;
+    }
     const int64_t need = (p.J + Sh::TEAMS - 1) / Sh::TEAMS;
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)num_sms() * occ));
     kernel<<<blocks, Sh::THREADS, smem, st>>>(p);
