@@ -3,7 +3,7 @@ tuning knobs are compile flags).
 
 Some kernels are compiled in several variants that give identical results
 with different launch shapes (see ftl_tune_variants in include/ftl.h): the
-FP32 draw on wrapped-diagonal trees (16 < R <= 32) descends 1, 2 or 3
+FP32 draw on wrapped-diagonal trees (16 < R <= 32) descends 1, 2 or 4
 samples per warp in lockstep.  Which is fastest depends on the GPU and the
 workload, so the tuner times every variant on a live sampler (CUDA events
 around the descent launches), selects the fastest for the current device

@@ -695,6 +695,112 @@ __device__ __forceinline__ void descend_d32_multi(const float *__restrict__ G, c
     }
 }
 
+// Four queries' forms at once: lane l passes its part of every form and gets
+// the sum over the warp of form l / 8 -- the sums of a butterfly over lane
+// distances 16, 8, 4, 2, 1 (warp_sum's), in fewer instructions.
+__device__ __forceinline__ float quad_reduce(const float (&p)[4], int lane) {
+    const bool up16 = (lane & 16) != 0, up8 = (lane & 8) != 0;
+    const float a = (up16 ? p[2] : p[0]) + __shfl_xor_sync(0xffffffffu, up16 ? p[0] : p[2], 16);
+    const float b = (up16 ? p[3] : p[1]) + __shfl_xor_sync(0xffffffffu, up16 ? p[1] : p[3], 16);
+    float v = (up8 ? b : a) + __shfl_xor_sync(0xffffffffu, up8 ? a : b, 8);
+    v += __shfl_xor_sync(0xffffffffu, v, 4);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    return v;
+}
+
+// descend_d32_multi for four queries: the lanes of group l / 8 carry sample
+// l / 8's state (dh, dl: its draw), so the reductions and decisions of the
+// four take the instructions of one.  cu, frac, mroot: of the lane's sample.
+template <class QF>
+__device__ __forceinline__ void descend_d32_quad(const float *__restrict__ G, const DGeom &g, float dh, float dl,
+                                                 const QF (&qf)[4], int lane, uint32_t &cu, float &frac,
+                                                 float &mroot) {
+    constexpr int S = kDiag32Stride;
+    cu = 0;
+    if (is_leaf(g, 0)) {
+        frac = fminf(dh + dl, 1.0f);
+        mroot = 1.0f;
+        return;
+    }
+    float th, tl, mP, mL;
+    {
+        float p[4];
+        const float4 *r4 = reinterpret_cast<const float4 *>(G), *l4 = reinterpret_cast<const float4 *>(G + S);
+        const float4 rv[4] = {__ldg(r4 + lane), __ldg(r4 + 32 + lane), __ldg(r4 + 64 + lane), __ldg(r4 + 96 + lane)};
+        const float4 lv[4] = {__ldg(l4 + lane), __ldg(l4 + 32 + lane), __ldg(l4 + 64 + lane), __ldg(l4 + 96 + lane)};
+        const float r16 = __ldg(G + 512 + lane), l16 = __ldg(G + S + 512 + lane);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) p[c] = qf[c].dot(rv, r16);
+        mroot = mP = quad_reduce(p, lane);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) p[c] = qf[c].dot(lv, l16);
+        mL = quad_reduce(p, lane);
+        th = dh * mP;
+        tl = fmaf(dl, mP, fmaf(dh, mP, -th));
+        const float s = th + tl;
+        tl = tl - (s - th);
+        th = s;
+    }
+    const uint32_t ncount = (uint32_t)g.node_count;
+    const int lf = (int)g.lfill_level;
+    for (int lvl = 0; lvl <= lf; ++lvl) {
+        const bool go = !(lvl == lf && 2u * cu + 1u >= ncount);
+        if (lvl == lf && !__any_sync(0xffffffffu, go)) break;
+        if (lvl > 0) {
+            const uint32_t next = go ? 2u * cu + 1u : 0u;
+            float4 v[4][4];
+            float v16[4], p[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const float *node = G + (size_t)__shfl_sync(0xffffffffu, next, 8 * c) * (size_t)S;
+                const float4 *n4 = reinterpret_cast<const float4 *>(node);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) v[c][q] = __ldg(n4 + 32 * q + lane);
+                v16[c] = __ldg(node + 512 + lane);
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) p[c] = qf[c].dot(v[c], v16[c]);
+            mL = quad_reduce(p, lane);
+        }
+        if (go) {
+            if (((th - mL) + tl) <= 0.0f) {
+                cu = 2u * cu + 1u;
+                mP = mL;
+            } else {
+                cu = 2u * cu + 2u;
+                df_sub(th, tl, mL);
+                mP = fmaxf(mP - mL, 0.0f);
+            }
+        }
+    }
+    const float f = mP > 0.0f ? (th + tl) / mP : 0.0f;
+    frac = fminf(fmaxf(f, 0.0f), 1.0f);
+}
+
+// The lockstep descents of NC queries, four by lane groups.
+template <int NC, class QF>
+__device__ __forceinline__ void descend_d32(const float *__restrict__ G, const DGeom &g, const float (&dh)[NC],
+                                            const float (&dl)[NC], const QF (&qf)[NC], int lane, uint32_t (&cu)[NC],
+                                            float (&frac)[NC], float (&mroot)[NC]) {
+    if constexpr (NC == 4) {
+        const bool g2 = (lane & 16) != 0, g1 = (lane & 8) != 0;
+        const float odh = g2 ? (g1 ? dh[3] : dh[2]) : (g1 ? dh[1] : dh[0]);
+        const float odl = g2 ? (g1 ? dl[3] : dl[2]) : (g1 ? dl[1] : dl[0]);
+        uint32_t ocu;
+        float ofrac, oroot;
+        descend_d32_quad(G, g, odh, odl, qf, lane, ocu, ofrac, oroot);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            cu[c] = __shfl_sync(0xffffffffu, ocu, 8 * c);
+            frac[c] = __shfl_sync(0xffffffffu, ofrac, 8 * c);
+            mroot[c] = __shfl_sync(0xffffffffu, oroot, 8 * c);
+        }
+    } else {
+        descend_d32_multi<NC>(G, g, dh, dl, qf, lane, cu, frac, mroot);
+    }
+}
+
 // ------------------------------------------------------------- leaf scan
 
 // The warp's staged query as per-lane registers (entry lane + 32q in [q]).

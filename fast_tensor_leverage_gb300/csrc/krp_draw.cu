@@ -227,7 +227,7 @@ __device__ __forceinline__ void draw_samples_d32(const DrawParams &p, int64_t i0
             dl[c] = __shfl_sync(0xffffffffu, ul[c], k);
         }
         const float *Ge = (const float *)p.eig_G + (size_t)k * (size_t)(2 * R - 1) * kDiag32Stride;
-        descend_d32_multi<NC>(Ge, p.eig, dh, dl, qf, lane, cu, frac, mroot);
+        descend_d32<NC>(Ge, p.eig, dh, dl, qf, lane, cu, frac, mroot);
         // Gram-tree descents, query h o W[u]
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
@@ -239,7 +239,7 @@ __device__ __forceinline__ void draw_samples_d32(const DrawParams &p, int64_t i0
             dl[c] = __shfl_sync(0xffffffffu, ul[c], N + k);
         }
         const DGeom &g = p.gram[k];
-        descend_d32_multi<NC>((const float *)p.gram_G[k], g, dh, dl, qf, lane, cu, frac, mroot);
+        descend_d32<NC>((const float *)p.gram_G[k], g, dh, dl, qf, lane, cu, frac, mroot);
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
             bool empty = false;
@@ -294,13 +294,19 @@ __global__ void __launch_bounds__(Blk<RMAX, T>::WARPS * 32, Resident<RMAX, T, fa
 
 // Block shape of the FP32 DIAG32 draw kernel per variant NC (samples a warp
 // descends in lockstep): warps per block and threads per SM its register
-// budget is set for.  NC = 1: 8 warps, 768 threads (85 registers); NC = 2
-// and 3: 4 warps, 512 threads (128 registers).  Which variant runs is the
-// autotuner's choice (ftl_tune_set), default NC = 3.
+// budget is set for.  NC = 1: 8 warps, 768 threads (85 registers); NC = 2: 4
+// warps, 512 threads (128 registers); NC = 4: 4 warps, 384 threads (168
+// registers), reductions and decisions by lane groups.  Which variant runs is
+// the autotuner's choice (ftl_tune_set).  Default: NC = 4 where the leaf blocks
+// are 32 x 32 and come from FP32 copies (N = 3, I = 2^23, R = 32, J = 50,000:
+// 0.770 ms per descent, NC = 1 0.852, NC = 3 without lane groups 0.788);
+// NC = 1 otherwise, where the scan of a leaf block is the longer part of a
+// mode and more warps overlap it better (R = 25, J = 65,536, two modes of
+// 300,600 rows: 0.49 ms against 0.53 with copies, 0.60 against 0.61 without).
 template <int NC, bool SW = false>
 struct D32Shape {
     static constexpr int WARPS = NC == 1 ? 8 : 4;
-    static constexpr int RESIDENT = SW ? (NC <= 3 ? 640 : NC == 4 ? 512 : 384) : (NC == 1 ? 768 : 512);
+    static constexpr int RESIDENT = SW ? (NC <= 3 ? 640 : NC == 4 ? 512 : 384) : (NC == 1 ? 768 : NC == 4 ? 384 : 512);
     static constexpr size_t SMEM = SW ? (size_t)WARPS * NC * kDiag32Stride * sizeof(float) : 0;
 };
 
@@ -645,7 +651,9 @@ static int launch_draw(const DrawParams &p, cudaStream_t st) {
             case 3: lrc = launch_d32<S32, 3, true>(p, st); break;
             case 4: lrc = launch_d32<S32, 4, true>(p, st); break;
             case 5: lrc = launch_d32<S32, 6, true>(p, st); break;
-            default: lrc = launch_d32<S32, 3, false>(p, st); break;
+            default:
+                lrc = S32 && p.R == 32 ? launch_d32<S32, 4, false>(p, st) : launch_d32<S32, 1, false>(p, st);
+                break;
         }
         if (lrc) return lrc;
     } else {

@@ -9,12 +9,13 @@
 // class of the family.  Unset entries use the family's default.
 //
 // Families:
-//   FTL_TUNE_DRAW: the FP32 draw on DIAG32 trees (16 < R <= 32); variants
-//     0, 1, 2 descend 1, 2, 3 samples per warp in lockstep with the query
-//     weights in registers (1: 8 warps per block, 768 threads per SM; 2 and
-//     3: 4 warps per block, 512 threads per SM); variants 3, 4, 5 keep the
-//     weights in shared memory and descend 3, 4, 6 samples per warp (640,
-//     512, 384 threads per SM).  Other ranks and precisions have one variant.
+//   FTL_TUNE_DRAW: the FP32 draw on DIAG32 trees (16 < R <= 32).  Variants 0
+//     and 1 descend 1 and 2 samples per warp in lockstep with the query weights
+//     in registers; variant 2, the default, 4 samples with their reductions
+//     and decisions by lane groups where R = 32 and FP32 factor copies exist,
+//     else variant 0's; variants 3, 4, 5 keep the weights in shared memory and
+//     descend 3, 4, 6 samples per warp.  Other ranks and precisions have one
+//     variant.
 #include <mutex>
 
 #include "ftl_common.cuh"
