@@ -193,6 +193,19 @@ __device__ __forceinline__ float d2f_rn(double x) {
     return __double2float_rn(x);
 }
 
+// d2f_rn without branches for zeros, FP64 subnormals and results in the normal
+// FP32 range; other inputs set `odd` and give an unspecified value.
+__device__ __forceinline__ float d2f_rn_normal(double x, bool &odd) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const unsigned e = (hi >> 20) & 0x7ffu;
+    unsigned r = __funnelshift_l(lo, (hi & 0x7fffffffu) - (896u << 20), 3);
+    const unsigned rest = lo & 0x1fffffffu;
+    r += rest + (r & 1u) > 0x10000000u ? 1u : 0u;  // above half, or half and odd
+    if (e == 0u) r = 0u;
+    odd |= e != 0u && e - 897u > 253u;
+    return __uint_as_float((hi & 0x80000000u) | r);
+}
+
 // (double)x for a finite x that is zero or normal, by integer operations: the
 // conversion runs on the FP64 pipe, where a warp instruction takes 64 cycles.
 __device__ __forceinline__ double f2d_exact(float x) {
