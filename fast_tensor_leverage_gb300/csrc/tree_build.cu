@@ -6,12 +6,8 @@
 // leaf_node(b), and every internal node is the elementwise sum of its two
 // children (parent = left + right, the reference's association).
 //
-// Work layout: one CTA loads LB leaf blocks into shared memory (converted to
-// the tree precision, columns zero-padded to a multiple of 4), then each
-// thread accumulates one 4x4 tile of the upper triangle of one block's Gram
-// over the block's rows (2 vector shared loads per 16 FMAs) and writes its
-// packed elements.  The HBM traffic is the read of U plus the write of the
-// leaf Grams; the internal levels are a second, purely elementwise pass.
+// The HBM traffic is the read of U plus the write of the leaf Grams; the
+// internal levels are a second, purely elementwise pass.
 #include <algorithm>
 #include <cstdio>
 #include <type_traits>
@@ -37,10 +33,14 @@ __device__ __forceinline__ T to_tree(double x) {
     else return x;
 }
 
+// Leaf Grams: LB leaf blocks are staged a row per warp (at R = 32 a row per half
+// warp), then the threads take the 4 x 4 tiles of the upper triangles in leaf
+// order.  Bound by the copies for FP32 and by the FP64 pipe for FP64.  Kept
+// where leaf_gram_kernel is the slower one (build_tree has the figures).
 template <typename T>
-__global__ void __launch_bounds__(256) leaf_gram_kernel(const double *__restrict__ U, int64_t n,
-                                                        int R, int RP, DGeom g, int LB,
-                                                        T *__restrict__ G, float *__restrict__ U32) {
+__global__ void __launch_bounds__(256) leaf_gram_rows_kernel(const double *__restrict__ U, int64_t n,
+                                                             int R, int RP, DGeom g, int LB,
+                                                             T *__restrict__ G, float *__restrict__ U32) {
     extern __shared__ __align__(32) unsigned char smem_raw[];
     T *Us = reinterpret_cast<T *>(smem_raw);  // LB x F x RP
     const int64_t F = g.F;
@@ -158,6 +158,203 @@ __global__ void __launch_bounds__(256) leaf_gram_kernel(const double *__restrict
     }
 }
 
+// One TC x TC tile (ta, tb) of a staged leaf block's Gram; DIAG: ta == tb, the
+// upper part only.
+template <typename T, int TC, bool DIAG, class Store>
+__device__ __forceinline__ void leaf_tile(const T *__restrict__ base, int F, int RP, int ta, int tb, Store store) {
+    T acc[TC][TC];
+#pragma unroll
+    for (int x = 0; x < TC; ++x)
+#pragma unroll
+        for (int y = 0; y < TC; ++y) acc[x][y] = T(0);
+    const T *pa = base + TC * ta, *pb = base + TC * tb;
+#pragma unroll(TC == 5 ? 1 : 2)
+    for (int r = 0; r < F; ++r) {
+        T a[TC], b[TC];
+        if constexpr (TC == 4) {  // RP is a multiple of 4: aligned vectors
+            using V = typename Vec4<T>::type;
+            const V va = *reinterpret_cast<const V *>(pa + r * RP), vb = *reinterpret_cast<const V *>(pb + r * RP);
+            a[0] = va.x, a[1] = va.y, a[2] = va.z, a[3] = va.w;
+            b[0] = vb.x, b[1] = vb.y, b[2] = vb.z, b[3] = vb.w;
+        } else {
+#pragma unroll
+            for (int x = 0; x < TC; ++x) a[x] = pa[r * RP + x];
+#pragma unroll
+            for (int y = 0; y < TC; ++y) b[y] = DIAG ? a[y] : pb[r * RP + y];
+        }
+#pragma unroll
+        for (int x = 0; x < TC; ++x)
+#pragma unroll
+            for (int y = DIAG ? x : 0; y < TC; ++y) acc[x][y] = fma(a[x], b[y], acc[x][y]);
+    }
+#pragma unroll
+    for (int x = 0; x < TC; ++x)
+#pragma unroll
+        for (int y = DIAG ? x : 0; y < TC; ++y) store(TC * ta + x, TC * tb + y, acc[x][y]);
+}
+
+// Leaf Grams: a CTA stages LB leaf blocks (consecutive rows of U, in the tree's
+// precision, columns zero padded to RP, a multiple of TC), then the threads
+// take the TC x TC tiles of the upper triangles, the LB nt tiles on the
+// diagonals first, padded to whole warps: a warp has tiles of one kind and
+// spends TC (TC + 1) / 2 multiply-adds per row on diagonal ones.  FP64 is bound
+// by the FP64 pipe's multiply-adds, so TC, LB and the block size are chosen by
+// how many of them are spent (leaf_shape): R = 25 takes 5 x 5 tiles and 340 per
+// row where 4 x 4 tiles of 28 columns took 448.  FP32 is bound by copies and
+// writes: the rows are read as one contiguous run, four loads in flight per
+// thread (a warp per row left 7 of 32 lanes idle at R = 25 and waited for each
+// load), and a DIAG32 node is put together in shared memory and written in
+// 16-byte vectors (its entries lie scattered over 2,176 bytes).
+template <typename T, int TC>
+__global__ void __launch_bounds__(512) leaf_gram_kernel(const double *__restrict__ U, int64_t n, int R, int RP, DGeom g,
+                                                        int LB, T *__restrict__ G, float *__restrict__ U32) {
+    extern __shared__ __align__(32) unsigned char smem_raw[];
+    T *Us = reinterpret_cast<T *>(smem_raw);  // LB x F x RP
+    const int F = (int)g.F;
+    const int P = packed_size(R);
+    const int S = node_stride(R, sizeof(T));
+    const int nt = RP / TC;
+    const bool diag32 = node_layout(R, sizeof(T)) == FTL_LAYOUT_DIAG32;
+    const int64_t leaf_count = (n + F - 1) / F;
+    const int64_t nbatch = (leaf_count + LB - 1) / LB;
+    const int nrows = LB * F, blk = F * RP;
+    float *nodes = reinterpret_cast<float *>(Us + ((nrows * RP + 3) & ~3));  // DIAG32: LB nodes
+    const int tid = threadIdx.x, nth = blockDim.x;
+    for (int e = tid; e < nrows * RP; e += nth) Us[e] = T(0);
+    if (diag32)
+        for (int e = tid; e < LB * kDiag32Stride; e += nth) nodes[e] = 0.0f;
+    const int ndiag = LB * nt, ndw = (ndiag + 31) / 32 * 32, noff = nt * (nt - 1) / 2;
+    const int step_r = nth / R, step_c = nth - step_r * R;
+
+    for (int64_t batch = blockIdx.x; batch < nbatch; batch += gridDim.x) {
+        const int64_t leaf0 = batch * LB, row0 = leaf0 * F;
+        const int rows = (int)min((int64_t)nrows, n - row0);
+        __syncthreads();
+        // the rows are contiguous in U: one value per thread and step
+        int r = tid / R, c = tid - r * R;
+        const double *src = U + row0 * R;
+        float *dst = U32 ? U32 + row0 * R : nullptr;
+        const int total = rows * R;
+        for (int e = tid; e < total; e += 4 * nth) {
+            double x[4];
+            T v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) x[u] = e + u * nth < total ? src[e + u * nth] : 0.0;
+            if constexpr (sizeof(T) == 4) {
+                // branch-free, so that the four loads stay together
+                bool odd = false;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) v[u] = d2f_rn_normal(x[u], odd);
+                if (odd) {
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) v[u] = d2f_rn(x[u]);
+                }
+            } else {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) v[u] = x[u];
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (e + u * nth < total) {
+                    if (sizeof(T) == 4 && dst) dst[e + u * nth] = (float)v[u];
+                    Us[r * RP + c] = v[u];
+                }
+                r += step_r;
+                c += step_c;
+                if (c >= R) {
+                    c -= R;
+                    ++r;
+                }
+            }
+        }
+        if (rows < nrows)  // the last batch: rows past n are zero
+            for (int e = rows * RP + tid; e < nrows * RP; e += nth) Us[e] = T(0);
+        __syncthreads();
+        for (int w = tid; w < ndw + LB * noff; w += nth) {
+            const bool on_diag = w < ndw;
+            int lb, ta, tb;
+            if (on_diag) {
+                lb = w / nt;
+                ta = tb = w - lb * nt;
+            } else {
+                lb = (w - ndw) / noff;
+                int rem = w - ndw - lb * noff;
+                ta = 0;
+                while (rem >= nt - 1 - ta) {
+                    rem -= nt - 1 - ta;
+                    ++ta;
+                }
+                tb = ta + 1 + rem;
+            }
+            const int64_t leaf = leaf0 + lb;
+            if (lb >= LB || leaf >= leaf_count) continue;
+            T *Gn = G + leaf_node(g, leaf) * (int64_t)S;
+            float *node = nodes + lb * kDiag32Stride;
+            auto store = [&](int a, int b, T v) {
+                if (a >= R || b >= R) return;
+                if (sizeof(T) == 4 && diag32) {
+                    node[diag32_pos(a, b)] = (float)v;
+                    if (b - a == 16) node[512 + b] = (float)v;  // the second copy
+                } else {
+                    Gn[packed_index(a, b, R)] = v;
+                }
+            };
+            if (on_diag) {
+                if (ta == 0 && !diag32)
+                    for (int e = P; e < S; ++e) Gn[e] = T(0);
+                leaf_tile<T, TC, true>(Us + lb * blk, F, RP, ta, tb, store);
+            } else {
+                leaf_tile<T, TC, false>(Us + lb * blk, F, RP, ta, tb, store);
+            }
+        }
+        if (sizeof(T) == 4 && diag32) {
+            __syncthreads();
+            const int nv = kDiag32Stride / 4;
+            for (int e = tid; e < LB * nv; e += nth) {
+                const int lb = e / nv, v = e - lb * nv;
+                const int64_t leaf = leaf0 + lb;
+                if (leaf < leaf_count)
+                    reinterpret_cast<float4 *>(G + leaf_node(g, leaf) * (int64_t)S)[v] =
+                        reinterpret_cast<const float4 *>(nodes)[e];
+            }
+        }
+    }
+}
+
+// Leaves per CTA, threads and shared memory for TC x TC tiles: among the LB
+// whose blocks fit, the one that spends the fewest multiply-add slots per
+// leaf (whole warps of diagonal and of other tiles), the larger on a tie; FP32
+// blocks stay below 44 KB, so that five CTAs per SM overlap copies and writes.
+// With 5 x 5 tiles the slots are those of the fullest of an SM's four parts (a
+// warp of off-diagonal tiles weighs 25 to 15 there): FP64 R = 25, 8e5 rows, 578
+// us against 660 us by the sum; with 4 x 4 tiles the sum is better (R = 28, 588
+// us against 629 us).
+struct LeafShape {
+    int LB, threads;
+    size_t smem;
+};
+static LeafShape leaf_shape(int R, int64_t F, int TC, size_t esize) {
+    const int nt = (R + TC - 1) / TC, RP = nt * TC, noff = nt * (nt - 1) / 2;
+    const bool diag32 = node_layout(R, (int)esize) == FTL_LAYOUT_DIAG32;
+    LeafShape best{1, 32, 0};
+    double cost = 0.0;
+    for (int LB = 1; LB <= 64; ++LB) {
+        const size_t smem = (((size_t)LB * F * RP + 3) / 4 * 4) * esize + (diag32 ? (size_t)LB * kDiag32Stride * 4 : 0);
+        if (LB > 1 && smem > (esize == 4 ? 44u : 100u) * 1024u) break;
+        const int wd = (LB * nt + 31) / 32, wo = (LB * noff + 31) / 32;
+        if (LB > 1 && wd + wo > 16) break;
+        int part[4] = {0, 0, 0, 0};
+        for (int w = 0; w < wd + wo; ++w) part[w & 3] += w < wd ? TC * (TC + 1) / 2 : TC * TC;
+        const int most = std::max(std::max(part[0], part[1]), std::max(part[2], part[3]));
+        const double c = (TC == 5 ? most : part[0] + part[1] + part[2] + part[3]) / (double)LB;
+        if (LB == 1 || c <= cost) {
+            best = LeafShape{LB, std::min(512, std::max(4, wd + wo) * 32), smem};
+            cost = c;
+        }
+    }
+    return best;
+}
+
 __device__ __forceinline__ float4 vadd(float4 a, float4 b) {
     return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
 }
@@ -251,28 +448,57 @@ static int build_impl(const double *U, int64_t n, int R, int64_t F, int prec, T 
         if (rc) return rc;
         return build_internal<T>(geom, R, G, st);
     }
-    const int P = packed_size(R);
-    const int RP = (R + 3) / 4 * 4;
-    const size_t blk_bytes = (size_t)F * RP * sizeof(T);
-    const int nt = RP / 4;
-    const int tiles = nt * (nt + 1) / 2;
-    // Leaves per CTA: fill the 256 threads with 4x4 tiles, bounded by shared memory.
-    int LB = std::max(1, 256 / tiles);
-    while (LB > 1 && (size_t)LB * blk_bytes > 112u * 1024u) --LB;
-    size_t smem = (size_t)LB * blk_bytes;
-    if (smem > 227 * 1024)
-        return fail(FTL_E_UNSUPPORTED, "tree_build: leaf block of %lld x %d needs %zu B of shared memory",
-                    (long long)F, R, smem);
-    rc = ensure_smem((const void *)leaf_gram_kernel<T>, smem, "leaf_gram_kernel");
+    // 5 x 5 tiles where they leave fewer padding columns than 4 x 4; FP32 is not
+    // bound by multiply-adds (R = 25: 145 us with 4 x 4, 195 us with 5 x 5)
+    const int TC = sizeof(T) == 8 && R % 5 == 0 && R % 4 != 0 ? 5 : 4;
+    const LeafShape sh = leaf_shape(R, F, TC, sizeof(T));
+    // Which leaf kernel: a whole tree of 2e7 values in us, rows kernel / tiles
+    // kernel.  FP64: R = 1 3134 / 870, 8 601 / 252, 16 529 / 410, 20 596 / 489,
+    // 25 777 / 578, 31 749 / 704, 32 683 / 724, 33 1043 / 790, 64 1441 / 1299,
+    // 100 2201 / 1994, 128 3061 / 2779.  FP32: R = 1 2327 / 655, 8 357 / 147, 16
+    // 230 / 261, 20 260 / 154, 25 214 / 145, 31 173 / 128, 32 130 / 175, 64 154 /
+    // 288, 128 240 / 266.  A block too large for the tiles kernel is left to the
+    // other, which needs less shared memory for wrapped-diagonal nodes.
+    if (R == 32 || (sizeof(T) == 4 && (R > 32 || (R > 8 && R <= 16))) || sh.smem > 227 * 1024) {
+        const int P = packed_size(R);
+        const int RP = (R + 3) / 4 * 4;
+        const size_t blk_bytes = (size_t)F * RP * sizeof(T);
+        const int nt = RP / 4;
+        const int tiles = nt * (nt + 1) / 2;
+        // Leaves per CTA: fill the 256 threads with 4x4 tiles, bounded by shared memory.
+        int LB = std::max(1, 256 / tiles);
+        while (LB > 1 && (size_t)LB * blk_bytes > 112u * 1024u) --LB;
+        size_t smem = (size_t)LB * blk_bytes;
+        if (smem > 227 * 1024)
+            return fail(FTL_E_UNSUPPORTED, "tree_build: leaf block of %lld x %d needs %zu B of shared memory",
+                        (long long)F, R, smem);
+        rc = ensure_smem((const void *)leaf_gram_rows_kernel<T>, smem, "leaf_gram_kernel");
+        if (rc) return rc;
+        int64_t nbatch = (geom.leaf_count + LB - 1) / LB;
+        // one wave of resident CTAs, each looping over batches: a grid larger
+        // than what fits at once leaves a partial second wave
+        int occ = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, leaf_gram_rows_kernel<T>, 256, smem) != cudaSuccess || occ < 1)
+            occ = 1;
+        int grid = (int)std::min<int64_t>(nbatch, (int64_t)num_sms() * occ);
+        leaf_gram_rows_kernel<T><<<grid, 256, smem, st>>>(U, n, R, RP, g, LB, G, U32);
+        rc = check_launch("leaf_gram_rows_kernel");
+        if (rc) return rc;
+        return build_internal<T>(geom, R, G, st);
+    }
+    auto kernel = leaf_gram_kernel<T, 4>;
+    if constexpr (sizeof(T) == 8)
+        if (TC == 5) kernel = leaf_gram_kernel<T, 5>;
+    rc = ensure_smem((const void *)kernel, sh.smem, "leaf_gram_kernel");
     if (rc) return rc;
-    int64_t nbatch = (geom.leaf_count + LB - 1) / LB;
+    int64_t nbatch = (geom.leaf_count + sh.LB - 1) / sh.LB;
     // one wave of resident CTAs, each looping over batches: a grid larger
     // than what fits at once leaves a partial second wave
     int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, leaf_gram_kernel<T>, 256, smem) != cudaSuccess || occ < 1)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, sh.threads, sh.smem) != cudaSuccess || occ < 1)
         occ = 1;
     int grid = (int)std::min<int64_t>(nbatch, (int64_t)num_sms() * occ);
-    leaf_gram_kernel<T><<<grid, 256, smem, st>>>(U, n, R, RP, g, LB, G, U32);
+    kernel<<<grid, sh.threads, sh.smem, st>>>(U, n, R, (R + TC - 1) / TC * TC, g, sh.LB, G, U32);
     rc = check_launch("leaf_gram_kernel");
     if (rc) return rc;
     return build_internal<T>(geom, R, G, st);
