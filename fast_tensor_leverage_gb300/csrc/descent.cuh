@@ -142,7 +142,7 @@ struct QForm {
     // is 8.3 KB (FP32): 17 vectors per lane, and with two in flight a level
     // cost nine dependent L2 round trips.  N = 4, R = 64, J = 32,768 FP32
     // draw: 7.24 ms with 2, 4.50 ms with 8 (640 threads per SM), 3.83 ms with
-    // all 17 (512 threads).  R <= 32 keeps 2: five or nine vectors, many warps.
+    // all 17 (512 threads).  R <= 32 keeps 2: two to nine vectors, many warps.
     static constexpr int LB = RMAX <= 32 ? 2 : (sizeof(T) == 8 ? 8 : (RMAX <= 64 ? 17 : 32));
 
     // acc + this lane's products of its vectors t0 .. t0 + LB - 1, in the
@@ -156,6 +156,11 @@ struct QForm {
             if (FULL || e0 + 32 * W * u < S) g[u] = __ldg(reinterpret_cast<const V *>(node + e0 + 32 * W * u));
 #pragma unroll
         for (int u = 0; u < LB; ++u) {
+            // past the node for every lane: leave, so that no multiply-add is
+            // issued (on the FP64 pipe one takes 64 cycles with any lane count;
+            // J = 16,384, N = 3, R = 64, FP64: 6.95 -> 6.09 ms; FP32, J = 32,768,
+            // R = 33: 1.33 -> 1.14 ms)
+            if (!FULL && RMAX > 32 && 32 * W * (t0 + u) >= S) break;
             if (FULL || e0 + 32 * W * u < S) {
                 T gv[W], xv[W];
                 Vec16<T>::get(g[u], gv);
@@ -179,8 +184,25 @@ struct QForm {
         return partial_of(node, s, S, lane);
     }
     static __device__ __forceinline__ T partial_of(const T *__restrict__ node, const T *s, int S, int lane) {
-        const int full = S / (32 * W);  // vectors every lane has
         T acc = T(0);
+        if constexpr (RMAX <= 32 && sizeof(T) == 8) {
+            // FP64-pipe bound: no multiply-add issued for vectors past the node
+            // (a warp instruction takes 64 cycles with any number of lanes)
+#pragma unroll 2
+            for (int e0 = 0; e0 < S; e0 += 32 * W) {
+                const int e = e0 + lane * W;
+                if (e < S) {
+                    T gv[W], xv[W];
+                    Vec16<T>::get(__ldg(reinterpret_cast<const V *>(node + e)), gv);
+                    Vec16<T>::get(*reinterpret_cast<const V *>(s + e), xv);
+#pragma unroll
+                    for (int w = 0; w < W; ++w) acc = fma(gv[w], xv[w], acc);
+                }
+            }
+            return acc;
+        }
+        if constexpr (LB >= NS::NV) return batch<false>(acc, node, s, S, 0, lane);
+        const int full = S / (32 * W);  // vectors every lane has
         int t = 0;
 #pragma unroll 1
         for (; t + LB <= full; t += LB) acc = batch<true>(acc, node, s, S, t, lane);
@@ -855,11 +877,13 @@ __device__ __forceinline__ T transpose_reduce(T (&v)[K], int lane) {
 // any use, and each chunk's K row dot products are finished by one
 // transpose-reduce.  xq holds the warp's query in the compute type.  A
 // selection past the last row of a partial block (only reachable when frac
-// rounds to >= 1) is clamped to that last row.
-template <int RMAX, typename T, typename UT = double>
-__device__ __forceinline__ int64_t leaf_scan(const UT *__restrict__ U, int R, const DGeom &g,
-                                             int64_t c, T frac, const LaneQuery<RMAX, T> &xq,
-                                             int lane, bool &empty) {
+// rounds to >= 1) is clamped to that last row.  FAST (FP32 trees on FP64 rows):
+// the rows are rounded to FP32 by integer operations; a value they do not
+// cover sets `odd`, and the result is then unspecified.
+template <int RMAX, typename T, typename UT, bool FAST>
+__device__ __forceinline__ int64_t leaf_scan_of(const UT *__restrict__ U, int R, const DGeom &g,
+                                                int64_t c, T frac, const LaneQuery<RMAX, T> &xq,
+                                                int lane, bool &empty, bool &odd) {
     constexpr int XPL = Shape<RMAX>::XPL;
     constexpr int K = FTL_DESC_LEAF_CHUNK;
     constexpr int LOGK = K == 8 ? 3 : (K == 16 ? 4 : 5);
@@ -869,25 +893,48 @@ __device__ __forceinline__ int64_t leaf_scan(const UT *__restrict__ U, int R, co
     const int64_t row0 = leaf * g.F;
     const int rows = (int)min((int64_t)F, g.n - row0);
     T q2[NCH];
-#pragma unroll
+#pragma unroll(FAST && NCH > 2 ? 1 : NCH)
     for (int ch = 0; ch < NCH; ++ch) {
         T v[K];
+        if constexpr (FAST) {
+            UT u[K][XPL];
 #pragma unroll
-        for (int rr = 0; rr < K; ++rr) {
-            const int r = K * ch + rr;
-            T acc = T(0);
-            if (r < rows) {
-                const UT *u = U + (row0 + r) * (int64_t)R;
+            for (int rr = 0; rr < K; ++rr) {
+                const int r = K * ch + rr;
+                const UT *ur = U + (row0 + r) * (int64_t)R;
 #pragma unroll
                 for (int q = 0; q < XPL; ++q) {
                     const int col = lane + 32 * q;
-                    if (col < R) acc = fma((T)__ldg(u + col), xq.v[q], acc);
+                    u[rr][q] = r < rows && col < R ? __ldg(ur + col) : UT(0);
                 }
             }
-            v[rr] = acc;
+#pragma unroll
+            for (int rr = 0; rr < K; ++rr) {
+                v[rr] = T(0);
+#pragma unroll
+                for (int q = 0; q < XPL; ++q) v[rr] = fma((T)d2f_rn_normal(u[rr][q], odd), xq.v[q], v[rr]);
+                if (K * ch + rr >= rows) v[rr] = T(0);
+            }
+        } else {
+#pragma unroll
+            for (int rr = 0; rr < K; ++rr) {
+                const int r = K * ch + rr;
+                T acc = T(0);
+                if (r < rows) {
+                    const UT *u = U + (row0 + r) * (int64_t)R;
+#pragma unroll
+                    for (int q = 0; q < XPL; ++q) {
+                        const int col = lane + 32 * q;
+                        if (col < R) acc = fma((T)__ldg(u + col), xq.v[q], acc);
+                    }
+                }
+                v[rr] = acc;
+            }
         }
-        T q = transpose_reduce<K, T>(v, lane);
-        q2[ch] = q * q;
+        const T q = transpose_reduce<K, T>(v, lane);
+#pragma unroll
+        for (int i = 0; i < NCH; ++i)
+            if (i == ch) q2[i] = q * q;
     }
     // Sequential prefix in row order (same association as the reference's
     // running sum); every lane walks the same sequence, lane r keeps row r's
@@ -975,6 +1022,38 @@ __device__ __forceinline__ int64_t leaf_scan(const UT *__restrict__ U, int R, co
     }
     if (res >= rows) res = rows - 1;
     return row0 + res;
+}
+
+template <int RMAX, typename T, typename UT, bool FAST>
+__device__ __noinline__ int64_t leaf_scan_call(const UT *U, int R, const DGeom &g, int64_t c, T frac,
+                                               LaneQuery<RMAX, T> xq, int lane, bool &empty, bool &odd) {
+    return leaf_scan_of<RMAX, T, UT, FAST>(U, R, g, c, frac, xq, lane, empty, odd);
+}
+
+// The scan of leaf_scan_of.  FP32 trees on FP64 rows: R conversions a row on the
+// FP64 pipe were the longer part of the scan where R is small; by integer
+// operations an update of CP-ALS at R = 25 (J = 65,536, two sampled modes) takes
+// 1.69 ms against 1.76, a draw at R = 28 (J = 32,768) 0.39 against 0.46, at R = 64
+// (four modes) 3.69 against 3.74.  R > 32 calls it, so that its 64 registers of
+// rows are not live with the descent's.  A block with an FP32-subnormal, huge or
+// non-finite value is scanned again with the hardware's conversion.  INT_CVT
+// false: the tree sampler at R <= 32, whose one scan per warp hides the
+// conversions (R = 16, J = 16,384: 61 us, 71 with the integer operations).
+template <int RMAX, typename T, typename UT = double, bool INT_CVT = true>
+__device__ __forceinline__ int64_t leaf_scan(const UT *__restrict__ U, int R, const DGeom &g,
+                                             int64_t c, T frac, const LaneQuery<RMAX, T> &xq,
+                                             int lane, bool &empty) {
+    constexpr bool FAST = INT_CVT && sizeof(T) == 4 && sizeof(UT) == 8;
+    bool odd = false;
+    if constexpr (FAST) {
+        int64_t t;
+        if constexpr (RMAX > 32) t = leaf_scan_call<RMAX, T, UT, true>(U, R, g, c, frac, xq, lane, empty, odd);
+        else t = leaf_scan_of<RMAX, T, UT, true>(U, R, g, c, frac, xq, lane, empty, odd);
+        if (__any_sync(0xffffffffu, odd)) t = leaf_scan_call<RMAX, T, UT, false>(U, R, g, c, frac, xq, lane, empty, odd);
+        return t;
+    } else {
+        return leaf_scan_of<RMAX, T, UT, false>(U, R, g, c, frac, xq, lane, empty, odd);
+    }
 }
 
 // Leaf row selection for R = F = 32 from the FP32 factor copy (the same

@@ -171,10 +171,12 @@ __device__ __forceinline__ void draw_sample(const DrawParams &p, int64_t i, Draw
 // Threads per SM the register budget of a draw kernel is set for: what the
 // warps' outer products leave room for in shared memory (R > 64: one block;
 // 32 < R <= 64: 16 warps in FP32, 12 in FP64), so that the node vectors a
-// warp has in flight get the registers.
+// warp has in flight get the registers.  FP32 R <= 16 has its own shapes (one
+// chunk of leaf rows, two node vectors): N = 3, J = 32,768, R = 5 / 16 take 296 /
+// 364 us at 64 registers, 358 / 415 in the shapes of R = 32 at 40 registers.
 template <int RMAX, typename T, bool DIAG>
 struct Resident {
-    static constexpr int F32 = RMAX <= 32 ? 1536 : (RMAX <= 64 ? 512 : 192);
+    static constexpr int F32 = RMAX <= 32 ? 1024 : (RMAX <= 64 ? 512 : 192);
     static constexpr int F64 = RMAX <= 32 ? 512 : (RMAX <= 64 ? 384 : 64);
     static constexpr int value = sizeof(T) == 8 ? F64 : (DIAG ? FTL_DESC_RESIDENT_D32 : F32);
 };
@@ -566,12 +568,12 @@ __global__ void __launch_bounds__(Blk<RMAX, T>::WARPS * 32, Resident<RMAX, T, DI
         int64_t c = descend<RMAX>((const T *)p.G, p.S, p.g, p.draws[i], qf, lane, frac,
                                   p.g.F > 1 ? p.U : nullptr, R);
         bool empty = false;
-        int64_t t = p.g.F > 1 ? leaf_scan<RMAX, T>(p.U, R, p.g, c, frac, lane_query<RMAX, T>(xT, R, lane), lane, empty)
+        int64_t t = p.g.F > 1 ? leaf_scan<RMAX, T, double, (RMAX > 32)>(p.U, R, p.g, c, frac, lane_query<RMAX, T>(xT, R, lane), lane, empty)
                               : leaf_index(p.g, c);
         if constexpr (sizeof(T) == 4) {
             if (empty) {  // FP32 descent ended in an all-zero block: redo it evaluating both children
                 c = descend_careful<RMAX>((const float *)p.G, p.S, p.g, p.draws[i], qf, lane, frac);
-                t = leaf_scan<RMAX, T>(p.U, R, p.g, c, frac, lane_query<RMAX, T>(xT, R, lane), lane, empty);
+                t = leaf_scan<RMAX, T, double, (RMAX > 32)>(p.U, R, p.g, c, frac, lane_query<RMAX, T>(xT, R, lane), lane, empty);
             }
         }
         if (lane == 0) p.samples[i] = (uint64_t)t;
@@ -733,12 +735,12 @@ static int dispatch_draw_f32(const DrawParams &p, cudaStream_t st) {
     const bool diag = node_layout(p.R, 4) == FTL_LAYOUT_DIAG32;
     if (shadows_ready(p)) {
         if (diag) return launch_draw<32, true, true>(p, st);
-        if (p.R <= 32) return launch_draw<32, true, false>(p, st);
+        if (p.R <= 16) return launch_draw<16, true, false>(p, st);
         if (p.R <= 64) return launch_draw<64, true, false>(p, st);
         return launch_draw<128, true, false>(p, st);
     }
     if (diag) return launch_draw<32, false, true>(p, st);
-    if (p.R <= 32) return launch_draw<32, false, false>(p, st);
+    if (p.R <= 16) return launch_draw<16, false, false>(p, st);
     if (p.R <= 64) return launch_draw<64, false, false>(p, st);
     return launch_draw<128, false, false>(p, st);
 }
@@ -750,6 +752,7 @@ static int dispatch_tree_sample(const TreeSampleParams &p, cudaStream_t st) {
     const int64_t RF = std::max<int64_t>(p.R, p.g.F);
     if constexpr (sizeof(T) == 4)
         if (node_layout(p.R, sizeof(T)) == FTL_LAYOUT_DIAG32 && RF <= 32) return launch_tree_sample<32, T, true>(p, st);
+    if (sizeof(T) == 4 && RF <= 16) return launch_tree_sample<16, T, false>(p, st);
     if (RF <= 32) return launch_tree_sample<32, T, false>(p, st);
     if (RF <= 64) return launch_tree_sample<64, T, false>(p, st);
     return launch_tree_sample<128, T, false>(p, st);
@@ -939,12 +942,12 @@ static int sample_packed(const ftl_krp_plan *const *plans, int n, const uint32_t
     const bool diag = node_layout(R, 4) == FTL_LAYOUT_DIAG32;
     if (s32) {
         if (diag) return launch_multi<32, float, true, true>(mp, st);
-        if (R <= 32) return launch_multi<32, float, true, false>(mp, st);
+        if (R <= 16) return launch_multi<16, float, true, false>(mp, st);
         if (R <= 64) return launch_multi<64, float, true, false>(mp, st);
         return launch_multi<128, float, true, false>(mp, st);
     }
     if (diag) return launch_multi<32, float, false, true>(mp, st);
-    if (R <= 32) return launch_multi<32, float, false, false>(mp, st);
+    if (R <= 16) return launch_multi<16, float, false, false>(mp, st);
     if (R <= 64) return launch_multi<64, float, false, false>(mp, st);
     return launch_multi<128, float, false, false>(mp, st);
 }
