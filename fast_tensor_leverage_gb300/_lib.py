@@ -138,6 +138,8 @@ SIGNATURES = {
     "ftl_krp_plan_sizes": ([_INT, _INT, _INT, _SZP, _SZP, _SZP, _SZP], _INT),
     "ftl_krp_compute_m": ([ctypes.POINTER(KRPPlan), _U32, _P], _INT),
     "ftl_krp_draw": ([ctypes.POINTER(KRPPlan), _U32, _P, _P, _P, _P, _U64, _U64, _P], _INT),
+    "ftl_krp_table_bytes": ([_INT, _I64, _INT, _SZP], _INT),
+    "ftl_krp_sample_table": ([ctypes.POINTER(KRPPlan), _U32, _P, _P, _P, _P, _U64, _U64, _P, _P], _INT),
     "ftl_krp_sample": ([ctypes.POINTER(KRPPlan), _U32, _P, _P, _P, _P, _U64, _U64, _P], _INT),
     "ftl_krp_draw_static": ([_INT, _INT, _I64, _INT, _P, _P, _P, _U32, _P, _P, _P, _P, _U64, _U64, _P], _INT),
     "ftl_fiber_keys": ([_P, _INT, _I64, _I64, _I64, _INT, _P, _INT, _P, _P], _INT),
@@ -232,6 +234,13 @@ def ws_bytes(name: str, *args) -> int:
     """Workspace size query: name is one of dedup / mttkrp_rows / gram / colnorm / fit / ..."""
     out = ctypes.c_size_t()
     call(f"ftl_{name}_workspace_bytes", *args, ctypes.byref(out))
+    return out.value
+
+
+def table_bytes(R: int, J: int, prec: int) -> int:
+    """Scratch bytes of ftl_krp_sample_table; 0: such draws use none."""
+    out = ctypes.c_size_t()
+    call("ftl_krp_table_bytes", R, J, prec, ctypes.byref(out))
     return out.value
 
 

@@ -12,8 +12,9 @@
 //            internal nodes = child sums, every node then o G_k(root).
 //
 // The eigensolver is a cyclic parallel-order (round-robin) two-sided Jacobi
-// method on a dense symmetric matrix in shared memory, one CTA per matrix,
-// rotations skipped when |a_pq| <= 2^-53 sqrt(|a_pp a_qq|) (the relative
+// method on a dense symmetric matrix in shared memory, one CTA per matrix (FP64
+// trees with R > 32: a cluster of 8 CTAs per matrix, the matrix in L2), rotations
+// skipped when |a_pq| <= 2^-53 sqrt(|a_pp a_qq|) (the relative
 // criterion of Demmel and Veselic), eigenpairs sorted ascending as LAPACK's
 // dsyev returns them.  Eigenvector signs are irrelevant downstream (only
 // outer products v v^T are used).

@@ -18,10 +18,6 @@ constexpr int kTabLevels = 12;        // Gram-tree levels at most
 constexpr int kTabNodes = 1 << kTabLevels;
 constexpr int64_t kTabMinJ = 16384;
 
-// Bytes of the table, which lies behind the packed pseudo-inverse in M.
-__host__ __device__ inline size_t cm_table_offset(int N, int R) {
-    return (cm_pinv64_offset(N, R) + node_stride(R, 8) + 1) / 2 * 2;
-}
 inline size_t table_bytes(int R, int esize) { return (kTabEig + (size_t)R * kTabNodes) * esize; }
 
 // Gram-tree levels worth tabulating for J samples: L levels cost R 2^L forms

@@ -793,9 +793,18 @@ extern "C" int ftl_krp_plan_sizes(int N, int R, int prec, size_t *eig_bytes, siz
     FTL_CHECK_ARG(valid_prec(prec), "ftl_krp_plan_sizes: bad precision");
     const int esize = prec_bytes(prec);
     if (eig_bytes) *eig_bytes = (size_t)N * (2 * R - 1) * node_stride(R, esize) * esize;
-    if (M_bytes) *M_bytes = cm_table_offset(N, R) * sizeof(double) + table_bytes(R, esize);
+    if (M_bytes) *M_bytes = (cm_pinv64_offset(N, R) + node_stride(R, 8)) * sizeof(double);
     if (lambda_bytes) *lambda_bytes = (size_t)(N + 1) * R * sizeof(double);
     if (pinv32_bytes) *pinv32_bytes = (size_t)node_stride(R, 4) * sizeof(float);
+    return FTL_OK;
+}
+
+extern "C" int ftl_krp_table_bytes(int R, int64_t J, int prec, size_t *bytes) {
+    FTL_CHECK_ARG(bytes && R >= 1 && R <= FTL_MAX_RANK && J >= 1, "ftl_krp_table_bytes: bad R=%d J=%lld", R,
+                  (long long)J);
+    FTL_CHECK_ARG(valid_prec(prec), "ftl_krp_table_bytes: bad precision");
+    const int esize = prec_bytes(prec);
+    *bytes = J < kTabMinJ || node_layout(R, esize) == FTL_LAYOUT_DIAG32 ? 0 : table_bytes(R, esize);
     return FTL_OK;
 }
 
@@ -812,9 +821,9 @@ extern "C" int ftl_krp_compute_m(const ftl_krp_plan *plan, uint32_t j, void *str
 static void fill_draw_params(DrawParams &p, const ftl_krp_plan *plan, uint32_t j, uint64_t *samples, double *h,
                              double *weights, const double *draws, uint64_t seed, uint64_t ctr);
 
-// table: the plan's M holds room for the mass table (ftl_krp_plan_sizes).
+// table: device scratch for the mass table (ftl_krp_table_bytes), null: none.
 static int krp_sample(const ftl_krp_plan *plan, uint32_t j, uint64_t *samples, double *h, double *weights,
-                      const double *draws, uint64_t seed, uint64_t ctr, bool table, void *stream) {
+                      const double *draws, uint64_t seed, uint64_t ctr, void *table, void *stream) {
     int rc = validate_plan(plan);
     if (rc) return rc;
     FTL_CHECK_ARG(samples != nullptr, "ftl_krp_sample: samples is NULL");
@@ -828,7 +837,7 @@ static int krp_sample(const ftl_krp_plan *plan, uint32_t j, uint64_t *samples, d
         const bool diag = plan->prec == FTL_PREC_FP32 && node_layout(plan->R, 4) == FTL_LAYOUT_DIAG32;
         if (p.tab_mode < p.N && !diag) {
             p.tab_levels = table_levels(p.gram[p.tab_mode], p.R, plan->J);
-            if (p.tab_levels) p.table = plan->M + cm_table_offset(p.N, p.R);
+            if (p.tab_levels) p.table = table;
         }
     }
     cudaStream_t st = (cudaStream_t)stream;
@@ -839,7 +848,14 @@ static int krp_sample(const ftl_krp_plan *plan, uint32_t j, uint64_t *samples, d
 extern "C" int ftl_krp_sample(const ftl_krp_plan *plan, uint32_t j, uint64_t *samples, double *h,
                               double *weights, const double *draws, uint64_t seed, uint64_t ctr,
                               void *stream) {
-    return krp_sample(plan, j, samples, h, weights, draws, seed, ctr, true, stream);
+    return krp_sample(plan, j, samples, h, weights, draws, seed, ctr, nullptr, stream);
+}
+
+extern "C" int ftl_krp_sample_table(const ftl_krp_plan *plan, uint32_t j, uint64_t *samples, double *h,
+                                    double *weights, const double *draws, uint64_t seed, uint64_t ctr,
+                                    void *table, void *stream) {
+    FTL_CHECK_ARG(aligned16(table), "ftl_krp_sample_table: the table must be 16-byte aligned");
+    return krp_sample(plan, j, samples, h, weights, draws, seed, ctr, table, stream);
 }
 
 static void fill_draw_params(DrawParams &p, const ftl_krp_plan *plan, uint32_t j, uint64_t *samples, double *h,
@@ -959,17 +975,6 @@ extern "C" int ftl_krp_draw(const ftl_krp_plan *plan, uint32_t j, uint64_t *samp
     if (rc) return rc;
     return ftl_krp_sample(plan, j, samples, h, weights, draws, seed, ctr, stream);
 }
-
-namespace ftl {
-// The static draw's plan (krp_draw_static.cu): M without room for the table.
-size_t static_M_bytes(int N, int R) { return (cm_pinv64_offset(N, R) + node_stride(R, 8)) * sizeof(double); }
-int static_draw(const ftl_krp_plan *plan, uint32_t j, uint64_t *samples, double *h, double *weights,
-                const double *draws, uint64_t seed, uint64_t ctr, void *stream) {
-    int rc = ftl_krp_compute_m(plan, j, stream);
-    if (rc) return rc;
-    return krp_sample(plan, j, samples, h, weights, draws, seed, ctr, false, stream);
-}
-}  // namespace ftl
 
 extern "C" int ftl_tree_sample(const void *G, int prec, const double *U, int64_t n, int R, int64_t F,
                                double *h, const double *scaled_h, uint64_t *samples,

@@ -28,12 +28,6 @@
 
 #include "ftl_common.cuh"
 
-namespace ftl {
-size_t static_M_bytes(int N, int R);
-int static_draw(const ftl_krp_plan *plan, uint32_t j, uint64_t *samples, double *h, double *weights,
-                const double *draws, uint64_t seed, uint64_t ctr, void *stream);
-}  // namespace ftl
-
 static __device__ __align__(256) unsigned char g_draw_scratch[FTL_DRAW_STATIC_SCRATCH_BYTES];
 
 namespace {
@@ -77,7 +71,6 @@ extern "C" int ftl_krp_draw_static(int N, int R, int64_t J, int prec, const int6
     size_t eig_b = 0, M_b = 0, lam_b = 0, p32_b = 0;
     int rc = ftl_krp_plan_sizes(N, R, prec, &eig_b, &M_b, &lam_b, &p32_b);
     if (rc) return rc;
-    M_b = ftl::static_M_bytes(N, R);  // no mass table: its room would shrink what fits the array
     const size_t off_M = align256(eig_b);
     const size_t off_lam = off_M + align256(M_b);
     const size_t off_p32 = off_lam + align256(lam_b);
@@ -108,5 +101,5 @@ extern "C" int ftl_krp_draw_static(int N, int R, int64_t J, int prec, const int6
     cudaError_t err = cudaMemsetAsync(base, 0, total, (cudaStream_t)stream);
     if (err != cudaSuccess)
         return ftl::fail(FTL_E_CUDA, "ftl_krp_draw_static: clearing scratch: %s", cudaGetErrorString(err));
-    return ftl::static_draw(&plan, j, samples_dev, h_dev, weights_dev, draws_dev, seed, ctr, stream);
+    return ftl_krp_draw(&plan, j, samples_dev, h_dev, weights_dev, draws_dev, seed, ctr, stream);
 }

@@ -15,6 +15,7 @@ struct ftl_sampler {
     ftl_krp_plan plan;
     int tree_prec;  // FTL_PREC_* the trees are built with (plan.prec is its node precision)
     int64_t F[FTL_MAX_MODES];
+    void *table;    // scratch of the draws' mass table, null: none
     std::vector<void *> owned;  // every cudaMalloc of this handle, freed by destroy
 };
 
@@ -82,7 +83,11 @@ extern "C" int ftl_sampler_create(int N, const int64_t *dims, int R, int64_t J, 
     }
     size_t eb = 0, mb = 0, lb = 0, pb = 0;
     if (rc == FTL_OK) rc = ftl_krp_plan_sizes(N, R, prec, &eb, &mb, &lb, &pb);
+    size_t tab = 0;
+    if (rc == FTL_OK) rc = ftl_krp_table_bytes(R, J, prec, &tab);
     void *e = nullptr, *m = nullptr, *l = nullptr, *q = nullptr;
+    s->table = nullptr;
+    if (rc == FTL_OK && tab) rc = alloc(s, tab, &s->table, false);
     if (rc == FTL_OK) rc = alloc(s, eb, &e, true);
     if (rc == FTL_OK) rc = alloc(s, mb, &m, true);
     if (rc == FTL_OK) rc = alloc(s, lb, &l, true);
@@ -131,7 +136,9 @@ extern "C" int ftl_sampler_draw(ftl_sampler *s, uint32_t j, uint64_t *samples_de
                                 double *weights_dev, const double *draws_dev, uint64_t seed, uint64_t ctr,
                                 void *stream) {
     FTL_CHECK_ARG(s, "ftl_sampler_draw: null pointer");
-    return ftl_krp_draw(&s->plan, j, samples_dev, h_dev, weights_dev, draws_dev, seed, ctr, stream);
+    const int rc = ftl_krp_compute_m(&s->plan, j, stream);
+    if (rc) return rc;
+    return ftl_krp_sample_table(&s->plan, j, samples_dev, h_dev, weights_dev, draws_dev, seed, ctr, s->table, stream);
 }
 
 extern "C" int ftl_sampler_destroy(ftl_sampler *s) {

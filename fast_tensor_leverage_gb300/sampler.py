@@ -72,6 +72,10 @@ class Sampler:
                                   torch.zeros(lam_b // 8, dtype=torch.float64, device=dev),
                                   torch.zeros(p32_b // 4, dtype=torch.float32, device=dev)))
         self.eig_G, self.M, self.lam, self.pinv32 = self._ws_sets[0]
+        # scratch of the descents' mass table, one per workspace set
+        tab_b = _lib.table_bytes(R, J, self._prec)
+        self._tables = [torch.empty(tab_b // 8, dtype=torch.float64, device=dev) if tab_b else None
+                        for _ in self._ws_sets]
         self.samples_dev = torch.zeros((N, J), dtype=torch.int64, device=dev)
         self.h_dev = torch.empty((J, R), dtype=torch.float64, device=dev)
         self.weights_dev = torch.empty(J, dtype=torch.float64, device=dev)
@@ -205,9 +209,7 @@ class Sampler:
         if self._overlap:
             main.wait_event(self._cm_done[b])
             ev0 = self._timing_event(main)
-            _lib.call("ftl_krp_sample", ctypes.byref(plan), j, self.samples_dev.data_ptr(),
-                      self.h_dev.data_ptr(), self.weights_dev.data_ptr(), d_ptr, self.seed,
-                      self.counter, int(main.cuda_stream))
+            self._descend(plan, b, j, d_ptr, main)
             self._timing_event(main, ev0)
             ev = torch.cuda.Event()
             ev.record(main)
@@ -220,12 +222,17 @@ class Sampler:
                 self._spec = (nb, j)
             self._last_j = j
         else:
-            _lib.call("ftl_krp_draw", ctypes.byref(plan), j, self.samples_dev.data_ptr(),
-                      self.h_dev.data_ptr(), self.weights_dev.data_ptr(), d_ptr, self.seed,
-                      self.counter, int(main.cuda_stream))
+            _lib.call("ftl_krp_compute_m", ctypes.byref(plan), j, int(main.cuda_stream))
+            self._descend(plan, 0, j, d_ptr, main)
         if d_ptr is None:
             self.counter += 2 * self.N * self.J
         return self.samples_dev, self.h_dev, self.weights_dev
+
+    def _descend(self, plan, b: int, j: int, d_ptr, main) -> None:
+        table = self._tables[b]
+        _lib.call("ftl_krp_sample_table", ctypes.byref(plan), j, self.samples_dev.data_ptr(),
+                  self.h_dev.data_ptr(), self.weights_dev.data_ptr(), d_ptr, self.seed,
+                  self.counter, table.data_ptr() if table is not None else None, int(main.cuda_stream))
 
     def _timing_event(self, stream, start=None):
         # records a timing event on `stream` when descent_events is a list;

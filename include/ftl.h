@@ -212,6 +212,17 @@ int ftl_krp_sample(const ftl_krp_plan *plan, uint32_t j, uint64_t *samples_dev,
                    double *h_dev, double *weights_dev, const double *draws_dev,
                    uint64_t seed, uint64_t ctr, void *stream);
 
+/* ftl_krp_sample with a scratch buffer of ftl_krp_table_bytes bytes (16-byte
+ * aligned device memory, used until the call's kernels are done) in which the
+ * upper levels of the first sampled mode, where all samples ask one of R + 1
+ * questions, are answered once per draw.  Same results.  table_dev NULL, or a
+ * draw that gains nothing by it: exactly ftl_krp_sample.  ftl_krp_table_bytes
+ * gives 0 where no draw of that kind would use the buffer. */
+int ftl_krp_table_bytes(int R, int64_t J, int prec, size_t *bytes);
+int ftl_krp_sample_table(const ftl_krp_plan *plan, uint32_t j, uint64_t *samples_dev,
+                         double *h_dev, double *weights_dev, const double *draws_dev,
+                         uint64_t seed, uint64_t ctr, void *table_dev, void *stream);
+
 /* Handle form of the sampler (EfficientKRPSampler, efficient_krp_sampler.hpp:
  * 32-75 for the state, :209-268 for KRPDrawSamples) for hosts that are not
  * Python: the handle owns the device factors, Gram trees and workspaces.
