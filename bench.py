@@ -520,7 +520,7 @@ def run_ours(args, ws, rank, local):
         "cpu_baseline": cpu,
         "one_mode_excluded": one_excluded,
         "autotune": {"family": "draw", "variant": tuning["variant"],
-                     "samples_per_warp": (1, 2, 3, 3, 4, 6)[tuning["variant"]] if tuning["ms"] else 1,
+                     "samples_per_warp": (1, 2, 4, 3, 4, 6)[tuning["variant"]] if tuning["ms"] else 1,
                      "weights_in_shared_memory": bool(tuning["ms"]) and tuning["variant"] >= 3,
                      "descent_ms_by_variant": {str(k): v for k, v in tuning["ms"].items()}},
         "accuracy": acc,

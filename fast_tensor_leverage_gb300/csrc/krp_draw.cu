@@ -304,7 +304,8 @@ __global__ void __launch_bounds__(Blk<RMAX, T>::WARPS * 32, Resident<RMAX, T, fa
 // 0.770 ms per descent, NC = 1 0.852, NC = 3 without lane groups 0.788);
 // NC = 1 otherwise, where the scan of a leaf block is the longer part of a
 // mode and more warps overlap it better (R = 25, J = 65,536, two modes of
-// 300,600 rows: 0.49 ms against 0.53 with copies, 0.60 against 0.61 without).
+// 300,600 rows: 0.49 ms against 0.53 with copies, 0.60 against 0.61
+// without, 0.56 since the rows are rounded by integer operations).
 template <int NC, bool SW = false>
 struct D32Shape {
     static constexpr int WARPS = NC == 1 ? 8 : 4;
