@@ -152,7 +152,7 @@ def estimate_bytes(req) -> int:
         for I in dims:   # FP64 factor (+ FP32 copy in FP32 mode) and tree
             total += I * R * (8 if prec == 0 else 12) + _lib.tree_bytes(I, min(R, I), R, prec)
         e, m, l, p = _lib.plan_sizes(N, R, prec)
-        return total + e + m + l + p + N * J * 8 + J * R * 8 + J * 8 + (1 << 20)
+        return total + e + m + l + p + _lib.table_bytes(R, J, prec) + N * J * 8 + J * R * 8 + J * 8 + (1 << 20)
     if isinstance(req, ALSRequest):
         N, R, J = len(req.dims), int(req.R), int(req.J)
         prec = _lib.PREC[req.precision]
@@ -166,7 +166,8 @@ def estimate_bytes(req) -> int:
         for I in req.dims:
             total += 2 * I * R * 8 + _lib.tree_bytes(I, min(R, I), R, prec)
         e, m, l, p = _lib.plan_sizes(N, R, prec)
-        return total + e + m + l + p + max(req.dims) * R * 8 + J * (N * 8 + R * 8 + 64) + (4 << 20)
+        return (total + e + m + l + p + _lib.table_bytes(R, J, prec) + max(req.dims) * R * 8
+                + J * (N * 8 + R * 8 + 64) + (4 << 20))
     raise TypeError(f"unknown request type {type(req).__name__}")
 
 
