@@ -142,8 +142,10 @@ struct QForm {
     // is 8.3 KB (FP32): 17 vectors per lane, and with two in flight a level
     // cost nine dependent L2 round trips.  N = 4, R = 64, J = 32,768 FP32
     // draw: 7.24 ms with 2, 4.50 ms with 8 (640 threads per SM), 3.83 ms with
-    // all 17 (512 threads).  R <= 32 keeps 2: two to nine vectors, many warps.
-    static constexpr int LB = RMAX <= 32 ? 2 : (sizeof(T) == 8 ? 8 : (RMAX <= 64 ? 17 : 32));
+    // all 17 (512 threads).  R <= 32: one at a time, one to nine vectors and many
+    // warps (R = 16, J = 32,768, N = 3, FP32: 326 us, 364 in batches of 2, which
+    // spilled).
+    static constexpr int LB = RMAX <= 32 ? 1 : (sizeof(T) == 8 ? 8 : (RMAX <= 64 ? 17 : 32));
 
     // acc + this lane's products of its vectors t0 .. t0 + LB - 1, in the
     // order of the elements; FULL: all of them lie inside the node
@@ -160,7 +162,7 @@ struct QForm {
             // issued (on the FP64 pipe one takes 64 cycles with any lane count;
             // J = 16,384, N = 3, R = 64, FP64: 6.95 -> 6.09 ms; FP32, J = 32,768,
             // R = 33: 1.33 -> 1.14 ms)
-            if (!FULL && RMAX > 32 && 32 * W * (t0 + u) >= S) break;
+            if (!FULL && 32 * W * (t0 + u) >= S) break;
             if (FULL || e0 + 32 * W * u < S) {
                 T gv[W], xv[W];
                 Vec16<T>::get(g[u], gv);
@@ -185,9 +187,9 @@ struct QForm {
     }
     static __device__ __forceinline__ T partial_of(const T *__restrict__ node, const T *s, int S, int lane) {
         T acc = T(0);
-        if constexpr (RMAX <= 32 && sizeof(T) == 8) {
-            // FP64-pipe bound: no multiply-add issued for vectors past the node
-            // (a warp instruction takes 64 cycles with any number of lanes)
+        if constexpr (RMAX <= 32) {
+            // no multiply-add issued for vectors past the node (on the FP64 pipe
+            // a warp instruction takes 64 cycles with any number of lanes)
 #pragma unroll 2
             for (int e0 = 0; e0 < S; e0 += 32 * W) {
                 const int e = e0 + lane * W;

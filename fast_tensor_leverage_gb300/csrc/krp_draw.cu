@@ -172,8 +172,8 @@ __device__ __forceinline__ void draw_sample(const DrawParams &p, int64_t i, Draw
 // warps' outer products leave room for in shared memory (R > 64: one block;
 // 32 < R <= 64: 16 warps in FP32, 12 in FP64), so that the node vectors a
 // warp has in flight get the registers.  FP32 R <= 16 has its own shapes (one
-// chunk of leaf rows, two node vectors): N = 3, J = 32,768, R = 5 / 16 take 296 /
-// 364 us at 64 registers, 358 / 415 in the shapes of R = 32 at 40 registers.
+// chunk of leaf rows, no spills): N = 3, J = 32,768, R = 5 / 16 take 276 / 326 us
+// at 64 registers; the shapes of R = 32 at 40 registers took 334 / 379.
 template <int RMAX, typename T, bool DIAG>
 struct Resident {
     static constexpr int F32 = RMAX <= 32 ? 1024 : (RMAX <= 64 ? 512 : 192);
