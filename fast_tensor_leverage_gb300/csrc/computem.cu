@@ -423,9 +423,9 @@ constexpr int kCmCluster = 8;
 constexpr int kCmClThreads = 512;
 
 struct CMClShared {
-    double cs[FTL_MAX_RANK + 2], lam[FTL_MAX_RANK];
+    double cs[2 * (FTL_MAX_RANK + 2)], lam[FTL_MAX_RANK];
     double V[FTL_MAX_RANK / kCmCluster * FTL_MAX_RANK];  // this CTA's rows of the eigenvectors
-    int pq[FTL_MAX_RANK + 2], order[FTL_MAX_RANK], flag;
+    int pq[2 * (FTL_MAX_RANK + 2)], order[FTL_MAX_RANK], flag;
 };
 
 // Eigenvalues from A's diagonal and their ascending order (sort_ascending's

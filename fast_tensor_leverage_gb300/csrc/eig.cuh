@@ -296,9 +296,14 @@ __device__ inline void jacobi64(double *A, double *V, int R, double *cs, int *pq
 // over all threads; every CTA forms all the round's rotations itself from the
 // same entries, so the CTAs agree on them without an exchange; a CTA keeps its
 // ceil(R / nr) rows of V in shared memory (Vs) and rotates them between
-// arriving at the barrier and waiting.  A0 holds the matrix; on return *eig
-// points to the copy with the eigenvalues on its diagonal and *vec to the
-// other one, which holds V.
+// arriving at the barrier and waiting.  The wait orders what came before the
+// arrivals, not these rotations of V, so a warp may form the next round's
+// rotations while another still reads this round's: they are kept in two sets
+// used in turn, and a set is written again two rounds later, behind the next
+// round's __syncthreads, which every reader of the set has reached.  Scratch:
+// cs (2 (R + 2) doubles), pq (2 (R + 2) ints), flag.  A0 holds the matrix; on
+// return *eig points to the copy with the eigenvalues on its diagonal and *vec
+// to the other one, which holds V.
 __device__ inline void jacobi64_cluster(double *A0, double *A1, int R, double *cs, int *pq, int *flag, double *Vs,
                                         int rk, int nr, double **eig, double **vec) {
     const int tid = threadIdx.x, nth = blockDim.x;
@@ -309,21 +314,25 @@ __device__ inline void jacobi64_cluster(double *A0, double *A1, int R, double *c
     cluster_sync();
     const int ntri = half * (half + 1) / 2;
     ClusterMat src{A0}, dst{A1};
+    int set = 0;
     for (int sweep = 0; sweep < 40; ++sweep) {
         for (int round = 0; round < n - 1; ++round) {
-            jacobi_rotations(src, R, round, cs, pq, flag);
+            double *c2 = cs + set * (R + 2);
+            int *p2 = pq + set * (R + 2);
+            set ^= 1;
+            jacobi_rotations(src, R, round, c2, p2, flag);
             __syncthreads();
             for (int w = rk + nr * tid; w < ntri; w += nr * nth) {  // every CTA the same share
                 int i, k;
                 jacobi_block(w, half, i, k);
-                jacobi_rotate(src, dst, R, i, k, cs, pq);
+                jacobi_rotate(src, dst, R, i, k, c2, p2);
             }
             asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
             for (int w = tid; w < half * nrows; w += nth) {
                 const int k = w / nrows, r = w - k * nrows;
-                const double ck = cs[2 * k], sk = cs[2 * k + 1];
+                const double ck = c2[2 * k], sk = c2[2 * k + 1];
                 if (sk == 0.0) continue;
-                const int pk = r * R + pq[2 * k], qk = r * R + pq[2 * k + 1];
+                const int pk = r * R + p2[2 * k], qk = r * R + p2[2 * k + 1];
                 const double vp = Vs[pk], vq = Vs[qk];
                 Vs[pk] = ck * vp - sk * vq;
                 Vs[qk] = sk * vp + ck * vq;
