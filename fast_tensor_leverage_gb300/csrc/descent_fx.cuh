@@ -6,9 +6,9 @@
 // cutoff.  A decision needs only the sign of draw * m - (mass left of the
 // cutoff).  Here that quantity is formed in fixed point, with a bound on its
 // error, and the decision is taken when it is larger than the bound; the
-// rare rest (and every query or tree with zeros, infinities or NaN where the
-// bound does not hold) is redone by the FP64 descent of descent.cuh.  So the
-// samples are the FP64 descent's.
+// rare rest (and every query or tree with infinities, NaN or a scale that the
+// bound does not hold for, see fx_in_range) is redone by the FP64 descent of
+// descent.cuh.  So the samples are the FP64 descent's.
 //
 // Arithmetic of a form sum_e g_e xx_e (g: node entries, xx: the weighted
 // outer product of the query, both scaled by powers of two so that the
@@ -51,7 +51,8 @@ __device__ __forceinline__ void pair_of(int e, int R, int &a, int &b) {
 
 // |v| 2^-q as h + l 2^-23, q such that FP64 exponent eb goes to FP32 exponent
 // 127 (kadj = -(eb - 127) << 20): h the upper 24 bits, l the next 23.  Values
-// below 2^-126 after scaling become about 2^-126.
+// below 2^-126 after scaling become about 2^-126, zeros and FP64 subnormals
+// among them, for eb >= 127 (fx_in_range; below, kadj > 0 would lift them).
 __device__ __forceinline__ void fx_split(uint32_t hi, uint32_t lo, int kadj, float &h, float &l) {
     const uint32_t sg = hi & 0x80000000u;
     const int a = __viaddmax_s32((int)(hi & 0x7fffffffu), kadj, 0x00100000);
@@ -181,6 +182,17 @@ __device__ __forceinline__ void fx_product(const float2 *xs, int a, int b, float
     pl = q - (ph - p);
 }
 
+// Whether queries whose largest FP64 exponent is emax may be scaled against
+// trees whose root's largest diagonal exponent is eg: both exponents are at
+// least 127 (fx_split), and the products x_a x_b and g x_a x_b of the largest
+// entries keep FP64's full precision, so that the FP64 forms are rounded sums
+// as the error bound takes them to be and neither lose bits in subnormals nor
+// overflow.
+__device__ __forceinline__ bool fx_in_range(int emax, int eg) {
+    const int x = emax - 1023, m = eg - 1023 + 2 * x;
+    return eg >= 127 && eg < 2046 && x >= -448 && x <= 480 && m >= -896 && m <= 960;
+}
+
 // Stage query x (FP64, XPL entries per lane, every warp of the team holds it)
 // for fx_eval against trees whose root's largest diagonal exponent is eg.
 // Returns false (uniformly) when the scaling does not hold.
@@ -209,7 +221,7 @@ __device__ __forceinline__ bool fx_stage(FxTeam<RMAX, TW> &tm, const double (&x)
         }
     }
     FxTeam<RMAX, TW>::sync();
-    if (emax == 0 || emax >= 2046 || eg <= 0 || eg >= 2046) return false;
+    if (!fx_in_range((int)emax, eg)) return false;
     const int P = packed_size(R);
     float bmax = 0.0f, b0 = 0.0f, b1 = 0.0f;
     for (int u = 0; u * ROW < tm.nvec; ++u) {
