@@ -147,20 +147,35 @@ __device__ inline void jacobi_eigen32(float *A, float *V, int R, float *csbuf, i
 // ten instructions of 64 cycles each; t comes from FP32 values scaled by a
 // common power of two, c from an FP32 reciprocal square root x of 1 + t^2 and
 // one third-order step, c = x + x e (1/2 + 3/8 e) with e = 1 - (1 + t^2) x^2
-// (the series of (1 - e)^(-1/2): 2^-22 becomes below 2^-60).
+// (the series of (1 - e)^(-1/2): 2^-22 becomes below 2^-60).  An entry below
+// 2^-100 of the largest of the three can still ask for a rotation (columns 30
+// decades apart and more); one of a_pp, a_qq is below 2^-94 of the other then,
+// t = a_pq / (a_qq - a_pp) to FP64 accuracy and the divisor is a normal FP32.
 __device__ __forceinline__ bool rotation64(double app, double aqq, double apq, double &c, double &s) {
     c = 1.0;
     s = 0.0;
     const int ep = (__double2hiint(app) >> 20) & 0x7ff, eq = (__double2hiint(aqq) >> 20) & 0x7ff,
               eo = (__double2hiint(apq) >> 20) & 0x7ff;
     const int em = max(max(ep, eq), eo);
-    if (eo == 0 || em >= 2047) return false;  // zero or subnormal entry, infinities, NaN
     const int sh = max(1, min(2045, 2046 - em));
     const double sc = __hiloint2double(sh << 20, 0);  // 2^(1023 - em): the largest in [1, 2)
     const double p = app * sc, q = aqq * sc, o = apq * sc;
-    if (!(o * o > 1.2325951644078309e-32 * fabs(p * q))) return false;  // 2^-106
-    const float d = d2f_rn(q - p), b = 2.0f * d2f_rn(o);
-    if (b == 0.0f) return false;
+    if (__builtin_expect(eo > max(0, em - 480) && em < 2047, 1)) {
+        if (!(o * o > 1.2325951644078309e-32 * fabs(p * q))) return false;  // 2^-106
+    } else {  // the squares could underflow; infinities
+        if (((__double2hiint(apq) & 0x7fffffff) | __double2loint(apq)) == 0) return false;
+        if (!(fabs(apq) > 1.1102230246251565e-16 * sqrt(fabs(app * aqq)))) return false;
+        if (em == 2047) {  // theta = 0
+            c = s = 0.70710678118654752;
+            return true;
+        }
+    }
+    const float d = d2f_rn(q - p);
+    if ((__double2hiint(o) & 0x7fffffff) < ((1023 - 100) << 20)) {
+        s = o * f2d_exact(1.0f / d);
+        return s != 0.0;
+    }
+    const float b = 2.0f * d2f_rn(o);
     const float tf = fabsf(b) / (fabsf(d) + sqrtf(fmaf(d, d, b * b)));  // theta = d / b
     const double t = f2d_exact((d < 0.0f) == (b < 0.0f) ? tf : -tf);
     const double w = fma(t, t, 1.0), x = f2d_exact(rsqrtf(fmaf(tf, tf, 1.0f)));
