@@ -1465,12 +1465,12 @@ extern "C" int ftl_weighted_gram(const double *lhs, const int32_t *rowidx, const
                                  double *gram_out, void *stream) {
     FTL_CHECK_ARG(lhs && workspace && gram_out, "ftl_weighted_gram: null pointer");
     FTL_CHECK_ARG(R >= 1 && R <= FTL_MAX_RANK, "ftl_weighted_gram: bad R=%d", R);
-    size_t need = 0;
-    ftl_gram_workspace_bytes(R, &need);
+    const int P = packed_size(R);
+    // one block per SM is enough (the size asked for before blocks shared an SM)
+    const size_t need = (size_t)num_sms() * P * sizeof(double);
     FTL_CHECK_ARG(ws_bytes >= need, "ftl_weighted_gram: workspace %zu < %zu bytes", ws_bytes, need);
     cudaStream_t st = (cudaStream_t)stream;
     const size_t smem = (size_t)(64 * R) * sizeof(double);
-    const int P = packed_size(R);
     int ept, threads;
     gram_shape(R, ept, threads);
     const auto kernel = ept == 1   ? gram_partial_kernel<1>
@@ -1483,7 +1483,8 @@ extern "C" int ftl_weighted_gram(const double *lhs, const int32_t *rowidx, const
     if (arc) return arc;
     int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem) != cudaSuccess || occ < 1) occ = 1;
-    const int nblk = num_sms() * std::min(occ, kGramBlocks);
+    const int nblk = (int)std::min<int64_t>((int64_t)num_sms() * std::min(occ, kGramBlocks),
+                                            (int64_t)(ws_bytes / (P * sizeof(double))));
     kernel<<<nblk, threads, smem, st>>>(lhs, rowidx, w, cnt, n_rows_dev, n_rows, R, (double *)workspace);
     gram_reduce_kernel<<<std::max(1, (P * 32 + 255) / 256), 256, 0, st>>>((const double *)workspace, nblk, R,
                                                                           gram_out);

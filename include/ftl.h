@@ -282,7 +282,9 @@ int ftl_dedup(const uint64_t *keys_dev, int64_t J, void *workspace, size_t ws_by
  * row(u) = rowidx ? rowidx[u] : u, s_u = (w ? w[row(u)] : 1) * (cnt ? cnt[u] : 1),
  * u < (n_rows_dev ? *n_rows_dev : n_rows).  Deterministic (fixed-order
  * reduction).  Replaces compute_pinv's Gram, cpp_ext/common.h:271-306, with
- * the sqrt(w) row scaling of cpp_ext/als.hpp:155-160 folded in. */
+ * the sqrt(w) row scaling of cpp_ext/als.hpp:155-160 folded in.
+ * ftl_gram_workspace_bytes gives the size at which several blocks share an SM;
+ * any size from a quarter of it on is taken, with fewer blocks. */
 int ftl_gram_workspace_bytes(int R, size_t *out);
 int ftl_weighted_gram(const double *lhs_dev, const int32_t *rowidx_dev, const double *w_dev,
                       const int32_t *cnt_dev, const int64_t *n_rows_dev, int64_t n_rows, int R,
