@@ -166,8 +166,14 @@ def estimate_bytes(req) -> int:
         for I in req.dims:
             total += 2 * I * R * 8 + _lib.tree_bytes(I, min(R, I), R, prec)
         e, m, l, p = _lib.plan_sizes(N, R, prec)
-        return (total + e + m + l + p + _lib.table_bytes(R, J, prec) + max(req.dims) * R * 8
-                + J * (N * 8 + R * 8 + 64) + (4 << 20))
+        # samples, rows, weights, keys and multiplicities of a draw, the solved
+        # rows and a sweep's uniforms; R x R matrices; the kernels' workspaces
+        # (the tensor keeps a Gram workspace of its own for the fit)
+        per_draw = J * (3 * N * 8 + 2 * R * 8 + 64) + (N + 3) * R * R * 8
+        work = (_lib.ws_bytes("dedup", J) + _lib.ws_bytes("mttkrp_rows", J, R) + 2 * _lib.ws_bytes("gram", R)
+                + _lib.ws_bytes("colnorm", R) + _lib.ws_bytes("fit"))
+        return (total + e + m + l + p + _lib.table_bytes(R, J, prec) + max(req.dims) * R * 8 + per_draw + work
+                + (4 << 20))
     raise TypeError(f"unknown request type {type(req).__name__}")
 
 
