@@ -1179,7 +1179,7 @@ struct KeyDigits {
 };
 
 template <int GW, int CPL, int NK>
-__global__ void __launch_bounds__(256) exact_mttkrp_rows_kernel(const int32_t *__restrict__ rrows,
+__global__ void __launch_bounds__(256) exact_mttkrp_rows_kernel(const uint32_t *__restrict__ rrows,
                                                                 const uint64_t *__restrict__ rkeys,
                                                                 const double *__restrict__ rvals, int64_t nnz,
                                                                 KeyDigits kd, int R, double *__restrict__ out) {
@@ -1194,23 +1194,24 @@ __global__ void __launch_bounds__(256) exact_mttkrp_rows_kernel(const int32_t *_
         double acc[CPL];
 #pragma unroll
         for (int c = 0; c < CPL; ++c) acc[c] = 0.0;
-        int32_t cur = -1;
+        int64_t cur = -1;
         auto flush = [&] {
 #pragma unroll
             for (int c = 0; c < CPL; ++c) {
                 const int col = gl + GW * c;
-                if (col < R) atomicAdd(out + (int64_t)cur * R + col, acc[c]);
+                if (col < R) atomicAdd(out + cur * R + col, acc[c]);
                 acc[c] = 0.0;
             }
         };
         for (int b = 0; b < EXM_RUN; b += GW) {
             const int64_t z = z0 + b + gl;
-            int32_t row = -1;
+            const int left = (int)max((int64_t)0, min((int64_t)GW, z1 - z0 - b));  // nonzeros of this step
+            uint32_t row = 0;
             double val = 0.0;
             uint32_t id[NK];
 #pragma unroll
             for (int k = 0; k < NK; ++k) id[k] = 0;
-            if (z < z1) {
+            if (gl < left) {
                 row = rrows[z];
                 val = rvals[z];
                 uint64_t key = rkeys[z];
@@ -1229,7 +1230,7 @@ __global__ void __launch_bounds__(256) exact_mttkrp_rows_kernel(const int32_t *_
             }
 #pragma unroll 1
             for (int g0 = 0; g0 < GW; g0 += G) {
-                int32_t hr[G];
+                uint32_t hr[G];
                 double pr[G][CPL], u0[G][CPL];  // value times the other factors' rows, and mode kd.U[0]'s row
 #pragma unroll
                 for (int g = 0; g < G; ++g) {
@@ -1248,7 +1249,7 @@ __global__ void __launch_bounds__(256) exact_mttkrp_rows_kernel(const int32_t *_
 #pragma unroll
                             for (int c = 0; c < CPL; ++c) {
                                 const int col = gl + GW * c;
-                                if (hr[g] >= 0 && col < R) {
+                                if (g0 + g < left && col < R) {
                                     if (k == 0) u0[g][c] = u[col];
                                     else pr[g][c] *= u[col];
                                 }
@@ -1258,8 +1259,8 @@ __global__ void __launch_bounds__(256) exact_mttkrp_rows_kernel(const int32_t *_
                 }
 #pragma unroll
                 for (int g = 0; g < G; ++g) {
-                    if (hr[g] >= 0) {
-                        if (hr[g] != cur) {
+                    if (g0 + g < left) {
+                        if ((int64_t)hr[g] != cur) {
                             if (cur >= 0) flush();
                             cur = hr[g];
                         }
@@ -1281,13 +1282,14 @@ static void launch_exact_rows(const int32_t *rrows, const uint64_t *rkeys, const
     const int64_t per_block = 8 * (32 / GW) * (int64_t)EXM_RUN;
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((nnz + per_block - 1) / per_block,
                                                                    (int64_t)num_sms() * 32));
+    const uint32_t *rows = (const uint32_t *)rrows;  // indices are uint32
     if (kd.n <= 2)
-        exact_mttkrp_rows_kernel<GW, CPL, 2><<<blocks, 256, 0, st>>>(rrows, rkeys, rvals, nnz, kd, R, out);
+        exact_mttkrp_rows_kernel<GW, CPL, 2><<<blocks, 256, 0, st>>>(rows, rkeys, rvals, nnz, kd, R, out);
     else if (kd.n <= 3)
-        exact_mttkrp_rows_kernel<GW, CPL, 3><<<blocks, 256, 0, st>>>(rrows, rkeys, rvals, nnz, kd, R, out);
+        exact_mttkrp_rows_kernel<GW, CPL, 3><<<blocks, 256, 0, st>>>(rows, rkeys, rvals, nnz, kd, R, out);
     else
         exact_mttkrp_rows_kernel<GW, CPL, FTL_MAX_MODES - 1>
-            <<<blocks, 256, 0, st>>>(rrows, rkeys, rvals, nnz, kd, R, out);
+            <<<blocks, 256, 0, st>>>(rows, rkeys, rvals, nnz, kd, R, out);
 }
 
 struct GramPtrs {

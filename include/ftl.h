@@ -417,7 +417,7 @@ int ftl_sparse_exact_mttkrp(const uint32_t *idx_dev, const double *vals_dev, int
 /* The same sum over the nonzeros sorted by their mode-j index (row_idx, with
  * fiber keys row_keys over tensor sizes dims, as ftl_fiber_keys forms them, and
  * values row_vals): one atomic add per column and row segment instead of one
- * per column and nonzero. */
+ * per column and nonzero.  row_idx holds the uint32 indices' bits. */
 int ftl_sparse_exact_mttkrp_rows(const int32_t *row_idx, const uint64_t *row_keys, const double *row_vals,
                                  int64_t nnz, int N, const int64_t *dims, int j,
                                  const double *const *U_dev, int R, double *out, int64_t I_j,
