@@ -1170,7 +1170,7 @@ __global__ void exact_mttkrp_kernel(const uint32_t *__restrict__ idx, const doub
 // changes -- instead of one per nonzero and column.  Bound by the FP64 pipe:
 // N - 1 multiply(-add)s per nonzero and group of lanes.  6.3e6 nonzeros of 3
 // modes at R = 25: 6.1 ms with an atomic per nonzero and column, 1.2 ms here.
-constexpr int EXM_RUN = 256;  // nonzeros per group and visit
+constexpr int EXM_RUN = 256;  // nonzeros per group and visit at most
 
 struct KeyDigits {
     int n;  // modes other than j, last first
@@ -1179,18 +1179,20 @@ struct KeyDigits {
 };
 
 template <int GW, int CPL, int NK>
-__global__ void __launch_bounds__(256) exact_mttkrp_rows_kernel(const uint32_t *__restrict__ rrows,
+__global__ void __launch_bounds__(256, CPL == 1 ? (NK <= 3 ? 5 : 4) : (CPL == 2 ? (NK <= 3 ? 4 : 3) : 2))
+    exact_mttkrp_rows_kernel(const uint32_t *__restrict__ rrows,
                                                                 const uint64_t *__restrict__ rkeys,
                                                                 const double *__restrict__ rvals, int64_t nnz,
-                                                                KeyDigits kd, int R, double *__restrict__ out) {
+                                                                KeyDigits kd, int R, int run,
+                                                                double *__restrict__ out) {
     constexpr int NG = 32 / GW, G = 4;
     const int lane = threadIdx.x & 31, gl = lane % GW;
     const int64_t gid = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * NG + lane / GW;
     const int64_t ngroups = (((int64_t)gridDim.x * blockDim.x) >> 5) * NG;
-    const int64_t nruns = (nnz + EXM_RUN - 1) / EXM_RUN;
+    const int64_t nruns = (nnz + run - 1) / run;
     const int64_t visits = (nruns + ngroups - 1) / ngroups;  // the same for every group: shuffles below
     for (int64_t vis = 0; vis < visits; ++vis) {
-        const int64_t z0 = (vis * ngroups + gid) * EXM_RUN, z1 = min(nnz, z0 + EXM_RUN);
+        const int64_t z0 = (vis * ngroups + gid) * run, z1 = min(nnz, z0 + run);
         double acc[CPL];
 #pragma unroll
         for (int c = 0; c < CPL; ++c) acc[c] = 0.0;
@@ -1203,7 +1205,7 @@ __global__ void __launch_bounds__(256) exact_mttkrp_rows_kernel(const uint32_t *
                 acc[c] = 0.0;
             }
         };
-        for (int b = 0; b < EXM_RUN; b += GW) {
+        for (int b = 0; b < run; b += GW) {
             const int64_t z = z0 + b + gl;
             const int left = (int)max((int64_t)0, min((int64_t)GW, z1 - z0 - b));  // nonzeros of this step
             uint32_t row = 0;
@@ -1279,17 +1281,23 @@ __global__ void __launch_bounds__(256) exact_mttkrp_rows_kernel(const uint32_t *
 template <int GW, int CPL>
 static void launch_exact_rows(const int32_t *rrows, const uint64_t *rkeys, const double *rvals, int64_t nnz,
                               const KeyDigits &kd, int R, double *out, cudaStream_t st) {
-    const int64_t per_block = 8 * (32 / GW) * (int64_t)EXM_RUN;
+    // Runs short enough that few nonzeros still spread over the chip: two blocks
+    // per SM (5,000 nonzeros in 3 modes, R = 8 / 64: 79 / 94 us in runs of 256, 14 /
+    // 24 us here; 300,000: 104 / 120, 27 / 93; an atomic per nonzero and column: 21 /
+    // 27, 192 / 476).
+    const int64_t groups = (int64_t)num_sms() * 16 * (32 / GW);
+    const int run = GW * (int)std::min<int64_t>(EXM_RUN / GW, (nnz + GW * groups - 1) / (GW * groups));
+    const int64_t per_block = 8 * (32 / GW) * (int64_t)run;
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((nnz + per_block - 1) / per_block,
                                                                    (int64_t)num_sms() * 32));
     const uint32_t *rows = (const uint32_t *)rrows;  // indices are uint32
     if (kd.n <= 2)
-        exact_mttkrp_rows_kernel<GW, CPL, 2><<<blocks, 256, 0, st>>>(rows, rkeys, rvals, nnz, kd, R, out);
+        exact_mttkrp_rows_kernel<GW, CPL, 2><<<blocks, 256, 0, st>>>(rows, rkeys, rvals, nnz, kd, R, run, out);
     else if (kd.n <= 3)
-        exact_mttkrp_rows_kernel<GW, CPL, 3><<<blocks, 256, 0, st>>>(rows, rkeys, rvals, nnz, kd, R, out);
+        exact_mttkrp_rows_kernel<GW, CPL, 3><<<blocks, 256, 0, st>>>(rows, rkeys, rvals, nnz, kd, R, run, out);
     else
         exact_mttkrp_rows_kernel<GW, CPL, FTL_MAX_MODES - 1>
-            <<<blocks, 256, 0, st>>>(rows, rkeys, rvals, nnz, kd, R, out);
+            <<<blocks, 256, 0, st>>>(rows, rkeys, rvals, nnz, kd, R, run, out);
 }
 
 struct GramPtrs {
