@@ -328,14 +328,21 @@ __global__ void __launch_bounds__(512) leaf_gram_kernel(const double *__restrict
 // With 5 x 5 tiles the slots are those of the fullest of an SM's four parts (a
 // warp of off-diagonal tiles weighs 25 to 15 there): FP64 R = 25, 8e5 rows, 578
 // us against 660 us by the sum; with 4 x 4 tiles the sum is better (R = 28, 588
-// us against 629 us).
+// us against 629 us).  Up to 32 leaves per SM the slots are those of the SM with
+// the most CTAs, at least one CTA's on one part, so that few leaves are spread
+// over the SMs: FP64 trees of 152 leaves, R = 30 / 56 / 80, 80 / 120 / 160 us ->
+// 53 / 55 / 93; 1,216 leaves, R = 40, 158 -> 104; 4,864 leaves, 375 -> 342.  Beyond
+// that the count of CTAs matters less than what they overlap (R = 36, 10,000
+// leaves: 502 us by slots per leaf, 550 by the fullest SM).
 struct LeafShape {
     int LB, threads;
     size_t smem;
 };
-static LeafShape leaf_shape(int R, int64_t F, int TC, size_t esize) {
+static LeafShape leaf_shape(int R, int64_t F, int64_t leaf_count, int TC, size_t esize) {
     const int nt = (R + TC - 1) / TC, RP = nt * TC, noff = nt * (nt - 1) / 2;
     const bool diag32 = node_layout(R, (int)esize) == FTL_LAYOUT_DIAG32;
+    const int sms = num_sms();
+    const bool few = leaf_count <= (int64_t)32 * sms;
     LeafShape best{1, 32, 0};
     double cost = 0.0;
     for (int LB = 1; LB <= 64; ++LB) {
@@ -346,7 +353,9 @@ static LeafShape leaf_shape(int R, int64_t F, int TC, size_t esize) {
         int part[4] = {0, 0, 0, 0};
         for (int w = 0; w < wd + wo; ++w) part[w & 3] += w < wd ? TC * (TC + 1) / 2 : TC * TC;
         const int most = std::max(std::max(part[0], part[1]), std::max(part[2], part[3]));
-        const double c = (TC == 5 ? most : part[0] + part[1] + part[2] + part[3]) / (double)LB;
+        const double all = TC == 5 ? 4 * most : part[0] + part[1] + part[2] + part[3];
+        const int64_t per_sm = ((leaf_count + LB - 1) / LB + sms - 1) / sms;  // CTAs on the fullest SM
+        const double c = few ? std::max(4.0 * most, all * (double)per_sm) : all / (double)LB;
         if (LB == 1 || c <= cost) {
             best = LeafShape{LB, std::min(512, std::max(4, wd + wo) * 32), smem};
             cost = c;
@@ -449,9 +458,10 @@ static int build_impl(const double *U, int64_t n, int R, int64_t F, int prec, T 
         return build_internal<T>(geom, R, G, st);
     }
     // 5 x 5 tiles where they leave fewer padding columns than 4 x 4; FP32 is not
-    // bound by multiply-adds (R = 25: 145 us with 4 x 4, 195 us with 5 x 5)
-    const int TC = sizeof(T) == 8 && R % 5 == 0 && R % 4 != 0 ? 5 : 4;
-    const LeafShape sh = leaf_shape(R, F, TC, sizeof(T));
+    // bound by multiply-adds (R = 25: 145 us with 4 x 4, 195 us with 5 x 5), nor are
+    // trees of one leaf per SM (R = 65, 152 leaves: 82 us with 5 x 5, rows kernel 74)
+    const int TC = sizeof(T) == 8 && R % 5 == 0 && R % 4 != 0 && geom.leaf_count > num_sms() ? 5 : 4;
+    const LeafShape sh = leaf_shape(R, F, geom.leaf_count, TC, sizeof(T));
     // Which leaf kernel: a whole tree of 2e7 values in us, rows kernel / tiles
     // kernel.  FP64: R = 1 3134 / 870, 8 601 / 252, 16 529 / 410, 20 596 / 489,
     // 25 777 / 578, 31 749 / 704, 32 683 / 724, 33 1043 / 790, 64 1441 / 1299,
@@ -459,7 +469,14 @@ static int build_impl(const double *U, int64_t n, int R, int64_t F, int prec, T 
     // 230 / 261, 20 260 / 154, 25 214 / 145, 31 173 / 128, 32 130 / 175, 64 154 /
     // 288, 128 240 / 266.  A block too large for the tiles kernel is left to the
     // other, which needs less shared memory for wrapped-diagonal nodes.
-    if (R == 32 || (sizeof(T) == 4 && (R > 32 || (R > 8 && R <= 16))) || sh.smem > 227 * 1024) {
+    // FP64 leaves much shorter than R are bound by the node writes, which the rows
+    // kernel makes in leaf order (20,000 leaves, F = 1: R = 25 80 / 91, 48 189 / 224,
+    // 128 1084 / 1326; F = R / 10: R = 20 70 / 76, 40 227 / 247, 80 913 / 926; at
+    // other ranks only single rows: R = 17 58 / 63, F = 2 67 / 69, R = 33 109 / 112,
+    // F = 2 137 / 125).
+    const bool short_leaves =
+        sizeof(T) == 8 && ((R % 5 == 0 && F * 10 <= R) || (R % 4 == 0 && F * 16 <= R) || (F == 1 && R >= 16));
+    if (R == 32 || (sizeof(T) == 4 && (R > 32 || (R > 8 && R <= 16))) || short_leaves || sh.smem > 227 * 1024) {
         const int P = packed_size(R);
         const int RP = (R + 3) / 4 * 4;
         const size_t blk_bytes = (size_t)F * RP * sizeof(T);
@@ -472,7 +489,7 @@ static int build_impl(const double *U, int64_t n, int R, int64_t F, int prec, T 
         if (smem > 227 * 1024)
             return fail(FTL_E_UNSUPPORTED, "tree_build: leaf block of %lld x %d needs %zu B of shared memory",
                         (long long)F, R, smem);
-        rc = ensure_smem((const void *)leaf_gram_rows_kernel<T>, smem, "leaf_gram_kernel");
+        rc = ensure_smem((const void *)leaf_gram_rows_kernel<T>, smem, "leaf_gram_rows_kernel");
         if (rc) return rc;
         int64_t nbatch = (geom.leaf_count + LB - 1) / LB;
         // one wave of resident CTAs, each looping over batches: a grid larger
