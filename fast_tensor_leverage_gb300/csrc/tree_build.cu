@@ -462,21 +462,27 @@ static int build_impl(const double *U, int64_t n, int R, int64_t F, int prec, T 
     // trees of one leaf per SM (R = 65, 152 leaves: 82 us with 5 x 5, rows kernel 74)
     const int TC = sizeof(T) == 8 && R % 5 == 0 && R % 4 != 0 && geom.leaf_count > num_sms() ? 5 : 4;
     const LeafShape sh = leaf_shape(R, F, geom.leaf_count, TC, sizeof(T));
-    // Which leaf kernel: a whole tree of 2e7 values in us, rows kernel / tiles
-    // kernel.  FP64: R = 1 3134 / 870, 8 601 / 252, 16 529 / 410, 20 596 / 489,
-    // 25 777 / 578, 31 749 / 704, 32 683 / 724, 33 1043 / 790, 64 1441 / 1299,
-    // 100 2201 / 1994, 128 3061 / 2779.  FP32: R = 1 2327 / 655, 8 357 / 147, 16
-    // 230 / 261, 20 260 / 154, 25 214 / 145, 31 173 / 128, 32 130 / 175, 64 154 /
-    // 288, 128 240 / 266.  A block too large for the tiles kernel is left to the
-    // other, which needs less shared memory for wrapped-diagonal nodes.
-    // FP64 leaves much shorter than R are bound by the node writes, which the rows
-    // kernel makes in leaf order (20,000 leaves, F = 1: R = 25 80 / 91, 48 189 / 224,
+    // Which leaf kernel: a whole tree in us, rows kernel / tiles kernel.  FP64, 2e7
+    // values: R = 1 3134 / 870, 8 601 / 252, 16 529 / 410, 20 596 / 489, 25 777 /
+    // 578, 31 749 / 704, 32 683 / 724, 33 1043 / 790, 64 1441 / 1299, 100 2201 /
+    // 1994, 128 3061 / 2779.  FP32 with the FP32 copy, 40,000 leaves: R = 1 48 / 37, 8
+    // 75 / 48, 9 79 / 53, 12 120 / 66, 16 154 / 91, 17 206 / 119, 20 227 / 135, 25 262 /
+    // 181, 31 309 / 221, 32 233 / 229, 33 334 / 258, 40 446 / 399, 48 658 / 508, 64
+    // 1036 / 869, 100 3099 / 2550; without the copy, 80,000 leaves: R = 9 107 / 64, 16
+    // 229 / 120, 32 393 / 405, 33 603 / 443, 64 1935 / 1578.  A block too large for the
+    // tiles kernel is left to the other, which needs less shared memory for
+    // wrapped-diagonal nodes.
+    // Leaves much shorter than R are bound by the node writes, which the rows kernel
+    // makes in leaf order (20,000 leaves; FP64, F = 1: R = 25 80 / 91, 48 189 / 224,
     // 128 1084 / 1326; F = R / 10: R = 20 70 / 76, 40 227 / 247, 80 913 / 926; at
     // other ranks only single rows: R = 17 58 / 63, F = 2 67 / 69, R = 33 109 / 112,
-    // F = 2 137 / 125).
+    // F = 2 137 / 125; FP32, F = 1: R = 33 68 / 79, 64 165 / 184, 128 471 / 545; F = 8:
+    // R = 40 108 / 116, 48 132 / 143, 64 184 / 180, 128 166 / 186; F = R / 4: R = 48
+    // 159 / 151, 64 144 / 135).
     const bool short_leaves =
-        sizeof(T) == 8 && ((R % 5 == 0 && F * 10 <= R) || (R % 4 == 0 && F * 16 <= R) || (F == 1 && R >= 16));
-    if (R == 32 || (sizeof(T) == 4 && (R > 32 || (R > 8 && R <= 16))) || short_leaves || sh.smem > 227 * 1024) {
+        sizeof(T) == 8 ? (R % 5 == 0 && F * 10 <= R) || (R % 4 == 0 && F * 16 <= R) || (F == 1 && R >= 16)
+                       : R > 32 && F * 5 <= R;
+    if (R == 32 || short_leaves || sh.smem > 227 * 1024) {
         const int P = packed_size(R);
         const int RP = (R + 3) / 4 * 4;
         const size_t blk_bytes = (size_t)F * RP * sizeof(T);

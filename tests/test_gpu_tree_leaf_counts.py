@@ -29,7 +29,11 @@ def ftl():
     (16, 1, 500), (15, 1, 500), (17, 1, 500), (17, 2, 400), (20, 2, 400), (20, 3, 400), (25, 2, 300), (25, 3, 300),
     (31, 1, 300), (33, 1, 300), (40, 4, 200), (40, 5, 200), (80, 8, 150), (80, 9, 150), (100, 10, 100), (100, 11, 100),
     (125, 12, 80), (48, 3, 200), (48, 4, 200), (64, 4, 150),
-    (64, 5, 150), (128, 8, 80), (128, 9, 80),
+    (64, 5, 150), (128, 8, 80), (128, 9, 80), (33, 6, 300), (33, 7, 300), (64, 12, 150),
+    (64, 13, 150), (128, 25, 60), (128, 26, 60),
+    # packed FP32 nodes on either side of the wrapped-diagonal ones
+    (9, 9, 4900), (12, 12, 300), (13, 13, 4864), (15, 15, 20), (16, 16, 4865), (34, 34, 700), (63, 63, 310), (64, 64, 160),
+    (96, 96, 20), (127, 127, 9), (128, 128, 40),
 ])
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
 def test_leaf_grams_match_oracle(ftl, R, F, leaves, precision):
