@@ -138,14 +138,12 @@ struct QForm {
         __syncwarp();
     }
 
-    // Node vectors a lane loads before it uses any of them.  A node of R = 64
-    // is 8.3 KB (FP32): 17 vectors per lane, and with two in flight a level
-    // cost nine dependent L2 round trips.  N = 4, R = 64, J = 32,768 FP32
-    // draw: 7.24 ms with 2, 4.50 ms with 8 (640 threads per SM), 3.83 ms with
-    // all 17 (512 threads).  R <= 32: one at a time, one to nine vectors and many
-    // warps (R = 16, J = 32,768, N = 3, FP32: 326 us, 364 in batches of 2, which
-    // spilled).
-    static constexpr int LB = RMAX <= 32 ? 1 : (sizeof(T) == 8 ? 8 : (RMAX <= 64 ? 17 : 32));
+    // R > 32: node vectors a lane loads before it uses any of them.  A node of R =
+    // 64 is 8.3 KB (FP32): 17 vectors per lane, and with two in flight a level
+    // cost nine dependent L2 round trips.  N = 4, R = 64, J = 32,768 FP32 draw:
+    // 7.24 ms with 2, 4.50 ms with 8 (640 threads per SM), 3.83 ms with all 17
+    // (512 threads).
+    static constexpr int LB = sizeof(T) == 8 ? 8 : (RMAX <= 64 ? 17 : 32);
 
     // acc + this lane's products of its vectors t0 .. t0 + LB - 1, in the
     // order of the elements; FULL: all of them lie inside the node
@@ -187,7 +185,22 @@ struct QForm {
     }
     static __device__ __forceinline__ T partial_of(const T *__restrict__ node, const T *s, int S, int lane) {
         T acc = T(0);
-        if constexpr (RMAX <= 32) {
+        if constexpr (RMAX <= 16 && sizeof(T) == 4) {
+            // one or two vectors per lane, loaded before any use (N = 3, R = 8, J =
+            // 1,000 / 100,000 draw: 45 / 717 us, one at a time 51 / 766)
+#pragma unroll
+            for (int t = 0; t < NS::NV; ++t) {
+                const int e = (lane + 32 * t) * W;
+                if (e < S) {
+                    T gv[W], xv[W];
+                    Vec16<T>::get(__ldg(reinterpret_cast<const V *>(node + e)), gv);
+                    Vec16<T>::get(*reinterpret_cast<const V *>(s + e), xv);
+#pragma unroll
+                    for (int w = 0; w < W; ++w) acc = fma(gv[w], xv[w], acc);
+                }
+            }
+            return acc;
+        } else if constexpr (RMAX <= 32) {
             // no multiply-add issued for vectors past the node (on the FP64 pipe
             // a warp instruction takes 64 cycles with any number of lanes)
 #pragma unroll 2
@@ -202,7 +215,12 @@ struct QForm {
                 }
             }
             return acc;
+        } else {
+            return batches(node, s, S, lane);
         }
+    }
+    static __device__ __forceinline__ T batches(const T *__restrict__ node, const T *s, int S, int lane) {
+        T acc = T(0);
         if constexpr (LB >= NS::NV) return batch<false>(acc, node, s, S, 0, lane);
         const int full = S / (32 * W);  // vectors every lane has
         int t = 0;
