@@ -179,6 +179,11 @@ struct Resident {
     static constexpr int F32 = RMAX <= 32 ? 1024 : (RMAX <= 64 ? 512 : 192);
     static constexpr int F64 = RMAX <= 32 ? 512 : (RMAX <= 64 ? 384 : 64);
     static constexpr int value = sizeof(T) == 8 ? F64 : (DIAG ? FTL_DESC_RESIDENT_D32 : F32);
+    // The tree sampler on packed FP32 nodes up to 32 columns: one descent and one
+    // scan per warp are short, and more warps hide them better (100,000 rows, J =
+    // 30,000; 1,024 threads per SM / 1,536: R = 8 79 / 67 us, R = 16 in leaves of 32
+    // rows 117 / 93).
+    static constexpr int tree = sizeof(T) == 4 && !DIAG && RMAX <= 32 ? 1536 : value;
 };
 
 // Samples i0 + c (c < NC, those below J) of one draw for FP32 trees in the
@@ -538,7 +543,7 @@ struct TreeSampleParams {
 // PartitionTree::PTSample_internal (cpp_ext/partition_tree.hpp:232-405):
 // x = scaled_h[i]; samples[i] = selected row; h[i] o= U[row].
 template <int RMAX, typename T, bool DIAG>
-__global__ void __launch_bounds__(Blk<RMAX, T>::WARPS * 32, Resident<RMAX, T, DIAG>::value / (Blk<RMAX, T>::WARPS * 32)) tree_sample_kernel(TreeSampleParams p) {
+__global__ void __launch_bounds__(Blk<RMAX, T>::WARPS * 32, Resident<RMAX, T, DIAG>::tree / (Blk<RMAX, T>::WARPS * 32)) tree_sample_kernel(TreeSampleParams p) {
     using S = Shape<RMAX>;
     constexpr int XPL = S::XPL;
     extern __shared__ __align__(16) unsigned char smem_raw[];
