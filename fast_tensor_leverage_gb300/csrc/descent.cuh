@@ -115,8 +115,8 @@ struct WarpSlot {
 // x^T G x for one query x against any node G (packed, node stride S): the
 // node is read as 16-byte vectors, vector v of lane l is v = l + 32 t, and
 // the matching weighted outer-product values live in the warp's shared-memory
-// slot.
-template <int RMAX, typename T>
+// slot.  BATCH: node vectors in flight (0: LB's default).
+template <int RMAX, typename T, int BATCH = 0>
 struct QForm {
     using NS = NodeShape<RMAX, T>;
     using V = typename Vec16<T>::type;
@@ -142,8 +142,8 @@ struct QForm {
     // 64 is 8.3 KB (FP32): 17 vectors per lane, and with two in flight a level
     // cost nine dependent L2 round trips.  N = 4, R = 64, J = 32,768 FP32 draw:
     // 7.24 ms with 2, 4.50 ms with 8 (640 threads per SM), 3.83 ms with all 17
-    // (512 threads).
-    static constexpr int LB = sizeof(T) == 8 ? 8 : (RMAX <= 64 ? 17 : 32);
+    // (512 threads); 6 and 640 threads where many warps are wanted (kNarrowBatch).
+    static constexpr int LB = BATCH ? BATCH : (sizeof(T) == 8 ? 8 : (RMAX <= 64 ? 17 : 32));
 
     // acc + this lane's products of its vectors t0 .. t0 + LB - 1, in the
     // order of the elements; FULL: all of them lie inside the node

@@ -22,19 +22,22 @@ int computem_launch(const ftl_krp_plan *plan, uint32_t j_norm, cudaStream_t st);
 int tuned_variant(int family, int R, int prec);
 int launch_draw_fx(const DrawParams &p, cudaStream_t st);
 
+// Node vectors in flight of the narrow draw kernel (launch_draw).
+constexpr int kNarrowBatch = 6;
+
 // Per-warp state of the draw kernels: the block's pair table and the warp's
 // shared-memory slot.
-template <int RMAX, typename T, bool DIAG = false>
+template <int RMAX, typename T, bool DIAG = false, bool NARROW = false>
 struct DrawWarp {
     const uint16_t *pairs;
     double *xd;
     T *xT;
-    typename QSel<RMAX, T, DIAG>::type qf;
+    std::conditional_t<NARROW, QForm<RMAX, T, kNarrowBatch>, typename QSel<RMAX, T, DIAG>::type> qf;
     int lane;
 };
 
-template <int RMAX, typename T, bool DIAG>
-__device__ __forceinline__ void setup_draw_warp(DrawWarp<RMAX, T, DIAG> &dw, unsigned char *smem_raw, int R, int P,
+template <int RMAX, typename T, bool DIAG, bool NARROW = false>
+__device__ __forceinline__ void setup_draw_warp(DrawWarp<RMAX, T, DIAG, NARROW> &dw, unsigned char *smem_raw, int R, int P,
                                                 int S) {
     uint16_t *pairs = (uint16_t *)smem_raw;
     build_pairs(pairs, R);
@@ -62,8 +65,8 @@ constexpr uint64_t kRedoSample = ~0ull;
 // Sample i of one draw: for every included mode the eigen-component descent
 // and the Gram-tree descent, then the weight and the row of h.  CAREFUL (FP32
 // fix-up pass only): both descents evaluate both children at every level.
-template <int RMAX, typename T, bool CAREFUL = false, bool S32 = false, bool DIAG = false>
-__device__ __forceinline__ void draw_sample(const DrawParams &p, int64_t i, DrawWarp<RMAX, T, DIAG> &dw) {
+template <int RMAX, typename T, bool CAREFUL = false, bool S32 = false, bool DIAG = false, bool NARROW = false>
+__device__ __forceinline__ void draw_sample(const DrawParams &p, int64_t i, DrawWarp<RMAX, T, DIAG, NARROW> &dw) {
     using S = Shape<RMAX>;
     constexpr int XPL = S::XPL;
     const int R = p.R;
@@ -128,8 +131,8 @@ __device__ __forceinline__ void draw_sample(const DrawParams &p, int64_t i, Draw
                 } else if (g.F > 1)
                     t = S32 ? leaf_scan<RMAX, T, float>(p.U32[k], R, g, c, frac, lane_query<RMAX, T>(xT, R, lane),
                                                         lane, empty)
-                            : leaf_scan<RMAX, T, double>(Uk, R, g, c, frac, lane_query<RMAX, T>(xT, R, lane), lane,
-                                                         empty);
+                            : leaf_scan<RMAX, T, double, !NARROW>(Uk, R, g, c, frac, lane_query<RMAX, T>(xT, R, lane),
+                                                                  lane, empty);
                 else
                     t = leaf_index(g, c);
                 // the careful pass (and FP64) keep what they found
@@ -183,6 +186,7 @@ struct Resident {
     // scan per warp are short, and more warps hide them better (100,000 rows, J =
     // 30,000; 1,024 threads per SM / 1,536: R = 8 79 / 67 us, R = 16 in leaves of 32
     // rows 117 / 93).
+    static constexpr int narrow = 640;  // the narrow draw kernel (launch_draw)
     static constexpr int tree = sizeof(T) == 4 && !DIAG && RMAX <= 32 ? 1536 : value;
 };
 
@@ -288,15 +292,17 @@ __device__ __forceinline__ void draw_samples_d32(const DrawParams &p, int64_t i0
     }
 }
 
-template <int RMAX, typename T, bool S32>
-__global__ void __launch_bounds__(Blk<RMAX, T>::WARPS * 32, Resident<RMAX, T, false>::value / (Blk<RMAX, T>::WARPS * 32)) krp_draw_kernel(DrawParams p) {
+template <int RMAX, typename T, bool S32, bool NARROW = false>
+__global__ void __launch_bounds__(Blk<RMAX, T>::WARPS * 32,
+                                  (NARROW ? Resident<RMAX, T, false>::narrow : Resident<RMAX, T, false>::value) /
+                                      (Blk<RMAX, T>::WARPS * 32)) krp_draw_kernel(DrawParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    DrawWarp<RMAX, T, false> dw;
-    setup_draw_warp<RMAX, T, false>(dw, smem_raw, p.R, p.P, p.S);
+    DrawWarp<RMAX, T, false, NARROW> dw;
+    setup_draw_warp<RMAX, T, false, NARROW>(dw, smem_raw, p.R, p.P, p.S);
     const int warp = threadIdx.x >> 5;
     for (int64_t i = (int64_t)blockIdx.x * Blk<RMAX, T>::WARPS + warp; i < p.J;
          i += (int64_t)gridDim.x * Blk<RMAX, T>::WARPS)
-        draw_sample<RMAX, T, false, S32, false>(p, i, dw);
+        draw_sample<RMAX, T, false, S32, false, NARROW>(p, i, dw);
 }
 
 // Block shape of the FP32 DIAG32 draw kernel per variant NC (samples a warp
@@ -667,11 +673,26 @@ static int launch_draw(const DrawParams &p, cudaStream_t st) {
     } else {
         const int trc = launch_table<RMAX>(p, st);
         if (trc) return trc;
-        const int arc = ensure_smem((const void *)krp_draw_kernel<RMAX, T, S32>, smem, "krp_draw_kernel");
+        auto kernel = krp_draw_kernel<RMAX, T, S32>;
+        // 32 < R <= 64: a sample's time is its levels' one after the other, so J
+        // samples take as long as their waves of resident warps.  16 warps per SM,
+        // each with a whole node in flight, are the faster ones for the same number of
+        // waves; the narrow kernel's 20 (six vectors, rows of FP64 factors converted by
+        // the hardware) where that is one wave less, and without copies up to R = 48.
+        // N = 3, 30,000 rows, wide / narrow, with FP32 copies: R = 33 J = 2,000 97 / 95
+        // us, 2,500 166 / 99, 40,000 1170 / 991; R = 64 178 / 185, 310 / 197, 2268 / 2046;
+        // without copies: R = 33 J = 50 104 / 93, 2,500 217 / 109, 40,000 1766 / 1132; R =
+        // 48 130 / 131, 271 / 159, 2180 / 1638; R = 64 162 / 182, 358 / 221, 2685 / 2406.
+        if constexpr (RMAX == 64) {
+            const int64_t sms = num_sms();
+            if ((p.J + 16 * sms - 1) / (16 * sms) > (p.J + 20 * sms - 1) / (20 * sms) || !(S32 || p.R > 48))
+                kernel = krp_draw_kernel<RMAX, T, S32, true>;
+        }
+        const int arc = ensure_smem((const void *)kernel, smem, "krp_draw_kernel");
         if (arc) return arc;
         int64_t blocks = (p.J + warps - 1) / warps;
         blocks = std::max<int64_t>(1, std::min<int64_t>(blocks, (int64_t)num_sms() * 64));
-        krp_draw_kernel<RMAX, T, S32><<<(unsigned)blocks, warps * 32, smem, st>>>(p);
+        kernel<<<(unsigned)blocks, warps * 32, smem, st>>>(p);
     }
     int rc = check_launch("krp_draw_kernel");
     if (rc) return rc;
