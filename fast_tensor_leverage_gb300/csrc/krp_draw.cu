@@ -675,17 +675,23 @@ static int launch_draw(const DrawParams &p, cudaStream_t st) {
         if (trc) return trc;
         auto kernel = krp_draw_kernel<RMAX, T, S32>;
         // 32 < R <= 64: a sample's time is its levels' one after the other, so J
-        // samples take as long as their waves of resident warps.  16 warps per SM,
-        // each with a whole node in flight, are the faster ones for the same number of
-        // waves; the narrow kernel's 20 (six vectors, rows of FP64 factors converted by
-        // the hardware) where that is one wave less, and without copies up to R = 48.
-        // N = 3, 30,000 rows, wide / narrow, with FP32 copies: R = 33 J = 2,000 97 / 95
-        // us, 2,500 166 / 99, 40,000 1170 / 991; R = 64 178 / 185, 310 / 197, 2268 / 2046;
-        // without copies: R = 33 J = 50 104 / 93, 2,500 217 / 109, 40,000 1766 / 1132; R =
-        // 48 130 / 131, 271 / 159, 2180 / 1638; R = 64 162 / 182, 358 / 221, 2685 / 2406.
+        // samples take as long as their waves of resident warps.  The wide kernel has
+        // 16 warps per SM, each with a whole node in flight; the narrow one 20, with six
+        // vectors, and rows of FP64 factors converted by the hardware.  Without FP32
+        // copies the narrow one is the faster up to R = 48, and above only where few
+        // waves become one less; with copies where it saves more than a sixth of the
+        // waves.  N = 3, one mode excluded, wide / narrow in us, factors of 3,000 /
+        // 400,000 rows: copies, R = 33, J = 2,800 116 / 72 and 141 / 83, 131,072 2198 /
+        // 1893 and 3661 / 3050; R = 64, J = 2,000 125 / 128 and 181 / 221, 2,800 220 / 136
+        // and 321 / 226, 14,000 611 / 555 and 941 / 1000, 131,072 4184 / 3679 and 6722 /
+        // 6421; no copies, R = 33, J = 2,000 101 / 75 and 120 / 88, 131,072 3589 / 2193 and
+        // 4419 / 3328; R = 48 4097 / 3042 and 5388 / 4931; R = 64, J = 5,500 344 / 275 and
+        // 491 / 441, 14,000 707 / 624 and 986 / 1058, 131,072 5043 / 4202 and 6645 / 6953
+        // (three modes of 65,536 rows 9680 / 10630).
         if constexpr (RMAX == 64) {
             const int64_t sms = num_sms();
-            if ((p.J + 16 * sms - 1) / (16 * sms) > (p.J + 20 * sms - 1) / (20 * sms) || !(S32 || p.R > 48))
+            const int64_t wide = (p.J + 16 * sms - 1) / (16 * sms), narrow = (p.J + 20 * sms - 1) / (20 * sms);
+            if (S32 ? 5 * wide > 6 * narrow : p.R <= 48 || (wide > narrow && narrow <= 3))
                 kernel = krp_draw_kernel<RMAX, T, S32, true>;
         }
         const int arc = ensure_smem((const void *)kernel, smem, "krp_draw_kernel");
