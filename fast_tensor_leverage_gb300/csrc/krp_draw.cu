@@ -316,7 +316,9 @@ __global__ void __launch_bounds__(Blk<RMAX, T>::WARPS * 32,
 // NC = 1 otherwise, where the scan of a leaf block is the longer part of a
 // mode and more warps overlap it better (R = 25, J = 65,536, two modes of
 // 300,600 rows: 0.49 ms against 0.53 with copies, 0.60 against 0.61
-// without, 0.56 since the rows are rounded by integer operations).
+// without, 0.56 since the rows are rounded by integer operations; R = 32 with
+// copies, three single-leaf trees of 20 rows, J = 1,000 / 50,000: 34 / 280 us
+// against 53 / 315).
 template <int NC, bool SW = false>
 struct D32Shape {
     static constexpr int WARPS = NC == 1 ? 8 : 4;
@@ -665,9 +667,12 @@ static int launch_draw(const DrawParams &p, cudaStream_t st) {
             case 3: lrc = launch_d32<S32, 3, true>(p, st); break;
             case 4: lrc = launch_d32<S32, 4, true>(p, st); break;
             case 5: lrc = launch_d32<S32, 6, true>(p, st); break;
-            default:
-                lrc = S32 && p.R == 32 ? launch_d32<S32, 4, false>(p, st) : launch_d32<S32, 1, false>(p, st);
+            default: {
+                bool leaves = true;  // every sampled tree is a single leaf
+                for (int k = 0; k < p.N; ++k) leaves = leaves && ((uint32_t)k == p.j || p.gram[k].node_count == 1);
+                lrc = S32 && p.R == 32 && !leaves ? launch_d32<S32, 4, false>(p, st) : launch_d32<S32, 1, false>(p, st);
                 break;
+            }
         }
         if (lrc) return lrc;
     } else {

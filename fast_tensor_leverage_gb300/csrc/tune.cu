@@ -12,8 +12,8 @@
 //   FTL_TUNE_DRAW: the FP32 draw on DIAG32 trees (16 < R <= 32).  Variants 0
 //     and 1 descend 1 and 2 samples per warp in lockstep with the query weights
 //     in registers; variant 2, the default, 4 samples with their reductions
-//     and decisions by lane groups where R = 32 and FP32 factor copies exist,
-//     else variant 0's; variants 3, 4, 5 keep the weights in shared memory and
+//     and decisions by lane groups where R = 32, FP32 factor copies exist and a
+//     sampled tree has more than one leaf, else variant 0's; variants 3, 4, 5 keep the weights in shared memory and
 //     descend 3, 4, 6 samples per warp.  Other ranks and precisions have one
 //     variant.
 #include <mutex>

@@ -579,7 +579,7 @@ int ftl_krp_sample_packed(const ftl_krp_plan *const *plans, int n, const uint32_
  * FTL_TUNE_DRAW: the FP32 draw on DIAG32 trees (16 < R <= 32); variants 0 and 1
  * descend 1 and 2 samples per warp in lockstep with the query weights in
  * registers, variant 2 (the default) 4 where R = 32 with FP32 factor copies and
- * 1 elsewhere, variants 3, 4, 5 descend 3, 4, 6 with the weights in shared
+ * a sampled tree of more than one leaf, 1 elsewhere, variants 3, 4, 5 descend 3, 4, 6 with the weights in shared
  * memory. */
 #define FTL_TUNE_DRAW 0
 int ftl_tune_variants(int family, int R, int prec, int *count, int *default_variant);
