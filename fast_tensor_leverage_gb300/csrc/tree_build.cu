@@ -478,11 +478,15 @@ static int build_impl(const double *U, int64_t n, int R, int64_t F, int prec, T 
     // other ranks only single rows: R = 17 58 / 63, F = 2 67 / 69, R = 33 109 / 112,
     // F = 2 137 / 125; FP32, F = 1: R = 33 68 / 79, 64 165 / 184, 128 471 / 545; F = 8:
     // R = 40 108 / 116, 48 132 / 143, 64 184 / 180, 128 166 / 186; F = R / 4: R = 48
-    // 159 / 151, 64 144 / 135).
+    // 159 / 151, 64 144 / 135; 100,000 leaves of one row at R = 16 89 / 100).  FP32, R
+    // = 57 .. 64: a leaf's tiles fill five warps, too few to copy its rows as fast as
+    // the rows kernel's eight where SMs have up to four leaves (R = 64, 304 leaves 32 /
+    // 34 us).
     const bool short_leaves =
         sizeof(T) == 8 ? (R % 5 == 0 && F * 10 <= R) || (R % 4 == 0 && F * 16 <= R) || (F == 1 && R >= 16)
-                       : R > 32 && F * 5 <= R;
-    if (R == 32 || short_leaves || sh.smem > 227 * 1024) {
+                       : (R > 32 && F * 5 <= R) || (R > 8 && R <= 16 && F <= 2);
+    const bool narrow_ctas = sizeof(T) == 4 && R > 56 && R <= 64 && geom.leaf_count <= (int64_t)4 * num_sms();
+    if (R == 32 || short_leaves || narrow_ctas || sh.smem > 227 * 1024) {
         const int P = packed_size(R);
         const int RP = (R + 3) / 4 * 4;
         const size_t blk_bytes = (size_t)F * RP * sizeof(T);

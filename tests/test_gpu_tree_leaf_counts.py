@@ -33,7 +33,8 @@ def ftl():
     (64, 13, 150), (128, 25, 60), (128, 26, 60),
     # packed FP32 nodes on either side of the wrapped-diagonal ones
     (9, 9, 4900), (12, 12, 300), (13, 13, 4864), (15, 15, 20), (16, 16, 4865), (34, 34, 700), (63, 63, 310), (64, 64, 160),
-    (96, 96, 20), (127, 127, 9), (128, 128, 40),
+    (96, 96, 20), (127, 127, 9), (128, 128, 40), (57, 57, 608), (57, 57, 609), (64, 64, 608), (64, 64, 609), (56, 56, 100),
+    (9, 2, 300), (9, 3, 300), (16, 2, 700), (16, 3, 700),
 ])
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
 def test_leaf_grams_match_oracle(ftl, R, F, leaves, precision):
