@@ -27,7 +27,7 @@
 #define FTL_DESC_PREFETCH 0        // L2 prefetch of next-level candidates (measured slower)
 #endif
 #ifndef FTL_DESC_EVAL2
-#define FTL_DESC_EVAL2 1           // root and first-level forms in one round trip
+#define FTL_DESC_EVAL2 1           // root and first-level forms reduced together
 #endif
 #ifndef FTL_DESC_LEAF_CHUNK
 #define FTL_DESC_LEAF_CHUNK 16     // leaf rows loaded per round trip (8, 16 or 32)
@@ -104,7 +104,7 @@ struct NodeShape {
 };
 
 // Per-warp shared-memory slot: the query in FP64 and in the compute type,
-// plus the packed outer product when it does not fit in registers.
+// plus the packed outer product (DIAG32 forms keep theirs in registers).
 template <int RMAX, typename T, bool DIAG = false>
 struct WarpSlot {
     static constexpr size_t xx_elems = DIAG ? 0 : NodeShape<RMAX, T>::SMAX;
@@ -233,7 +233,9 @@ struct QForm {
         return warp_sum(partial(node, lane));
     }
 
-    // Two independent forms with interleaved loads (one memory round trip).
+    // Two independent forms, their warp reductions interleaved.  Up to R = 32 the
+    // inlined sums leave the loads free to overlap; above, the two calls follow
+    // each other.
     __device__ __forceinline__ void eval2(const T *__restrict__ na, const T *__restrict__ nb,
                                           int lane, T &ra, T &rb) const {
         T acc_a = partial(na, lane), acc_b = partial(nb, lane);

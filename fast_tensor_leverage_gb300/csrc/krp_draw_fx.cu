@@ -4,17 +4,16 @@
 // those are certain, from the FP64 code of descent.cuh where they are not.
 // The FP64 work left per sample is h o W[u], the update of h and the weight.
 //
-// Measured (one GB300; FP64 forms before, this kernel now): N = 3, I = 2^22,
-// R = 32, J = 50,000, one mode excluded 6.25 -> 2.24 ms; N = 4, I = 1000,
-// R = 8, J = 10,000 with copies to the host 0.93 -> 0.20 ms.  It is bound by
-// the integer pipe (cutting the FP64 values, 46% of its peak) and the latency
-// of the node reads.
+// Measured (one GB300; FP64 forms before, this kernel with its mass table now):
+// N = 3, I = 2^22, R = 32, J = 50,000, one mode excluded 6.25 -> 1.66 ms; N = 4, I =
+// 1000, R = 8, J = 10,000 with copies to the host 0.93 -> 0.19 ms.  It is bound by
+// issue (60% of the slots at I = 2^20, R = 32; the integer pipe, which cuts the
+// FP64 values, 49% of its peak) and the latency of the node reads.
 //
 // One warp per sample up to R = 64 (at R = 32 a query's outer product takes
 // 4.2 KB of shared memory; 32 warps of 64 registers per SM measured 3% faster
-// than 24 of 80); above, a team of four
-// warps shares one sample, since a query of R = 100 takes 40 KB and one warp
-// per sample would leave five warps on an SM.
+// than 24 of 80); above, a team of four warps shares one sample, since a query of
+// R = 100 takes 40 KB and one warp per sample would leave five warps on an SM.
 #include <algorithm>
 
 #include "descent_fx.cuh"

@@ -36,7 +36,8 @@ __device__ __forceinline__ T to_tree(double x) {
 // Leaf Grams: LB leaf blocks are staged a row per warp (at R = 32 a row per half
 // warp), then the threads take the 4 x 4 tiles of the upper triangles in leaf
 // order.  Bound by the copies for FP32 and by the FP64 pipe for FP64.  Kept
-// where leaf_gram_kernel is the slower one (build_tree has the figures).
+// where leaf_gram_kernel is the slower one: R = 32, leaves much shorter than R, few
+// leaves at 56 < R <= 64 in FP32 (build_impl has the figures).
 template <typename T>
 __global__ void __launch_bounds__(256) leaf_gram_rows_kernel(const double *__restrict__ U, int64_t n,
                                                              int R, int RP, DGeom g, int LB,
